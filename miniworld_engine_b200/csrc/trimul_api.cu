@@ -116,7 +116,7 @@ int sm_count() {
 // attribute call is not free and these entry points sit on latency-sensitive host paths.
 bool ensure_smem_once(const void* fn, int bytes) {
     struct Entry { const void* fn; uint64_t devices; };
-    static Entry table[32];
+    static Entry table[64];
     static int used = 0;
     static std::mutex mu;
     int dev = 0;
@@ -127,7 +127,7 @@ bool ensure_smem_once(const void* fn, int bytes) {
         if (table[i].fn == fn) e = &table[i];
     if (e != nullptr && dev < 64 && ((e->devices >> dev) & 1u)) return true;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
-    if (e == nullptr && used < 32) { e = &table[used++]; e->fn = fn; e->devices = 0; }
+    if (e == nullptr && used < 64) { e = &table[used++]; e->fn = fn; e->devices = 0; }
     if (e != nullptr && dev < 64) e->devices |= 1ull << dev;
     return true;
 }
@@ -232,10 +232,10 @@ int launch_status() { return cudaGetLastError() == cudaSuccess ? TRIMUL_OK : TRI
 // predecessor has completed, so launch latency and set-up disappear from the critical path.  Every
 // kernel launched this way executes that wait before it touches global memory.
 template <typename... KArgs, typename... Args>
-int launch_stage(void (*kernel)(KArgs...), int grid, int block, int smem, cudaStream_t st, bool overlap,
+int launch_stage(void (*kernel)(KArgs...), dim3 grid, int block, int smem, cudaStream_t st, bool overlap,
                  Args&&... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid, 1, 1);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)block, 1, 1);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
@@ -251,6 +251,16 @@ inline bool overlap_launches(uint32_t flags) { return (flags & TRIMUL_FLAG_SERIA
 // ---------------------------------------------------------------------------------------
 // stage 1
 // ---------------------------------------------------------------------------------------
+// Positions per thread of the CUDA-core stages 1 and 3 (`groups` blocks share a position tile): the largest tile
+// that still gives `want` blocks.  Stage 1 wants two blocks on every SM (N = 96, c = 128: 70 us with 64 positions
+// per block, 95 with 128), stage 3 one and a half (N = 128: 67 us with 128 positions, 77 with 64; N = 96: 44 us
+// with 64, 55 with 32), its smaller tiles paying more shared-memory reads per FMA.
+int plain_positions_per_thread(int64_t pos, int groups, int64_t want) {
+    for (int tm = 8; tm > 2; tm /= 2)
+        if ((pos + 16 * tm - 1) / (16 * tm) * groups >= want) return tm;
+    return 2;
+}
+
 template <typename T>
 int run_plain_tm1(const trimul_desc* d, const void* z, const uint8_t* mask, const trimul_weights* w,
                   const trimul_planes* a, const trimul_planes* b, cudaStream_t st) {
@@ -262,9 +272,18 @@ int run_plain_tm1(const trimul_desc* d, const void* z, const uint8_t* mask, cons
     p.gamma = w->ln_in_weight; p.beta = w->ln_in_bias; p.eps = d->eps_in;
     p.w_left = w->w_left; p.w_left_gate = w->w_left_gate; p.w_right = w->w_right; p.w_right_gate = w->w_right_gate;
     p.a = view_of(*a); p.b = view_of(*b);
-    const int64_t grid = (int64_t)d->B * d->rows * ((d->N + kPlainPos - 1) / kPlainPos);
-    plain_tm1_kernel<T><<<(unsigned)grid, kPlainThreads, 0, st>>>(static_cast<const T*>(z), p);
-    return launch_status();
+    const int64_t pos = (int64_t)d->B * d->rows * d->N;
+    const int groups = 2 * ((d->c_hidden + kPlainCh - 1) / kPlainCh);
+    auto launch = [&](auto kernel, int tile_pos, int smem, int max_smem) {
+        if (!ensure_smem(kernel, max_smem)) return (int)TRIMUL_E_CUDA;
+        const dim3 grid((unsigned)((pos + tile_pos - 1) / tile_pos), (unsigned)groups);
+        return launch_stage(kernel, grid, kPlainThreads, smem, st, overlap_launches(d->flags), static_cast<const T*>(z), p);
+    };
+    switch (plain_positions_per_thread(pos, groups, 2 * (int64_t)sm_count())) {
+        case 8: return launch(plain_tm1_kernel<T, 8>, 128, plain_tm1_smem<8>(d->c), plain_tm1_smem<8>(kPlainMaxC));
+        case 4: return launch(plain_tm1_kernel<T, 4>, 64, plain_tm1_smem<4>(d->c), plain_tm1_smem<4>(kPlainMaxC));
+        default: return launch(plain_tm1_kernel<T, 2>, 32, plain_tm1_smem<2>(d->c), plain_tm1_smem<2>(kPlainMaxC));
+    }
 }
 
 // Warp-MMA kernels: bf16, c and h multiples of 16, weight matrices 32-byte aligned (fragment loads).
@@ -477,10 +496,18 @@ int run_wide_tm1(const trimul_desc* d, const void* z, const uint8_t* mask, const
 // ---------------------------------------------------------------------------------------
 template <typename T>
 int run_plain_contract(int planes, const trimul_planes* a, const trimul_planes* b, const trimul_planes* t,
-                       cudaStream_t st) {
-    dim3 grid((unsigned)((b->rows + 31) / 32), (unsigned)((a->rows + 31) / 32), (unsigned)planes);
-    plain_contract_kernel<T><<<grid, 256, 0, st>>>(view_of(*a), view_of(*b), view_of(*t));
-    return launch_status();
+                       cudaStream_t st, uint32_t flags) {
+    auto tiles = [&](int64_t n) { return ((b->rows + n - 1) / n) * ((a->rows + n - 1) / n); };
+    auto launch = [&](auto kernel, int n) {
+        const dim3 grid((unsigned)((b->rows + n - 1) / n), (unsigned)((a->rows + n - 1) / n), (unsigned)planes);
+        return launch_stage(kernel, grid, kPlainThreads, 0, st, overlap_launches(flags), view_of(*a), view_of(*b),
+                            view_of(*t));
+    };
+    // 128 x 128 tiles need half the shared-memory reads per FMA of 64 x 64 ones: taken when they fill the chip twice and
+    // pad the planes by less than a quarter more
+    if (planes * tiles(128) >= 2 * (int64_t)sm_count() && 4 * 4 * tiles(128) <= 5 * tiles(64))
+        return launch(plain_contract_kernel<T, 8>, 128);
+    return launch(plain_contract_kernel<T, 4>, 64);
 }
 
 bool fast_contract_ok(const trimul_planes* a, const trimul_planes* b, const trimul_planes* t, bool pair) {
@@ -561,10 +588,20 @@ int run_plain_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri,
     p.w_gate = w->w_gate; p.w_out = w->w_out;
     p.tri = view_of(*tri);
     p.drop_scale = desc_drop_scale(d);
-    const int64_t grid = (int64_t)d->B * d->rows * ((d->N + kPlainPos - 1) / kPlainPos);
-    plain_tm2_kernel<T><<<(unsigned)grid, kPlainThreads, 0, st>>>(static_cast<const T*>(z), static_cast<T*>(out),
-                                                                   static_cast<const T*>(residual), p);
-    return launch_status();
+    const int64_t pos = (int64_t)d->B * d->rows * d->N;
+    const int groups = (d->c + kPlainCh - 1) / kPlainCh;
+    auto launch = [&](auto kernel, int tile_pos, int smem, int max_smem) {
+        if (!ensure_smem(kernel, max_smem)) return (int)TRIMUL_E_CUDA;
+        const dim3 grid((unsigned)((pos + tile_pos - 1) / tile_pos), (unsigned)groups);
+        return launch_stage(kernel, grid, kPlainThreads, smem, st, overlap_launches(d->flags), static_cast<const T*>(z),
+                            static_cast<T*>(out), static_cast<const T*>(residual), p);
+    };
+    constexpr int kC = kPlainMaxC;
+    switch (plain_positions_per_thread(pos, groups, 3 * (int64_t)sm_count() / 2)) {
+        case 8: return launch(plain_tm2_kernel<T, 8>, 128, plain_tm2_smem<8>(d->c, d->c_hidden), plain_tm2_smem<8>(kC, kC));
+        case 4: return launch(plain_tm2_kernel<T, 4>, 64, plain_tm2_smem<4>(d->c, d->c_hidden), plain_tm2_smem<4>(kC, kC));
+        default: return launch(plain_tm2_kernel<T, 2>, 32, plain_tm2_smem<2>(d->c, d->c_hidden), plain_tm2_smem<2>(kC, kC));
+    }
 }
 
 int run_wmma_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri, const trimul_weights* w, void* out,
@@ -816,14 +853,14 @@ int trimul_b200_contract(int32_t dtype, uint32_t flags, int32_t planes, const tr
     if ((rc = check_planes(tri, a->rows, b->rows)) != TRIMUL_OK) return rc;
     if (a->rows <= 0 || b->rows <= 0 || a->cols <= 0) return TRIMUL_E_INVALID;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (dtype == TRIMUL_DTYPE_FP32) return run_plain_contract<float>(planes, a, b, tri, st);
+    if (dtype == TRIMUL_DTYPE_FP32) return run_plain_contract<float>(planes, a, b, tri, st, flags);
     if ((flags & TRIMUL_FLAG_PLAIN_KERNELS) == 0) {
         const bool pair = (flags & TRIMUL_FLAG_SINGLE_CTA_CONTRACT) == 0 && sm_count() >= 2;
         if (fast_contract_ok(a, b, tri, pair)) return run_fast_contract(planes, a, b, tri, st, status, pair, flags);
         if (pair && fast_contract_ok(a, b, tri, false))
             return run_fast_contract(planes, a, b, tri, st, status, false, flags);
     }
-    return run_plain_contract<__nv_bfloat16>(planes, a, b, tri, st);
+    return run_plain_contract<__nv_bfloat16>(planes, a, b, tri, st, flags);
 }
 
 namespace {
