@@ -803,6 +803,68 @@ __device__ __forceinline__ void ln_rows_warp(uint8_t* tile, int sub_bytes, int r
     }
 }
 
+// The same for rows of 64 channels with FOUR lanes per row: lane l works on row row0 + 8 i + (l >> 2) and owns 16-byte
+// chunks (l & 3) and (l & 3) + 4, i.e. 16 channels (gb: gamma pairs of the two chunks, then beta pairs, see
+// ln_load_affine_quad).  Half as many steps per warp as with eight lanes, and one shuffle stage less.  Odd rows
+// take their second chunk first, so that the eight lanes of a quarter warp (two rows) touch eight different 16-byte
+// columns of the swizzled tile.
+template <int kIters>
+__device__ __forceinline__ void ln_rows64_warp(uint8_t* tile, int row0, int lane, const f32x2 (&gb)[16], float eps,
+                                               uint32_t zero_bits) {
+    const int rr = lane >> 2;
+    const uint32_t j = (uint32_t)lane & 3u;
+    const bool odd = rr & 1;
+    constexpr float kInvC = 1.0f / 64.0f;
+#pragma unroll 2
+    for (int i = 0; i < kIters; ++i) {
+        const int r = row0 + 8 * i + rr;            // row0 is a multiple of 8: r & 7 == rr
+        uint8_t* rowp = tile + (uint32_t)r * 128u;
+        const uint32_t off0 = ((j ^ (uint32_t)rr) & 7u) << 4, off1 = (((j + 4u) ^ (uint32_t)rr) & 7u) << 4;
+        const uint4 va = *reinterpret_cast<const uint4*>(rowp + (odd ? off1 : off0));
+        const uint4 vb = *reinterpret_cast<const uint4*>(rowp + (odd ? off0 : off1));
+        const uint4 v0 = odd ? vb : va, v1 = odd ? va : vb;
+        const float shift = bf16_lo(__shfl_sync(0xffffffffu, v0.x, lane & 28));    // the row's channel 0
+        const f32x2 ns = f2_pack(-shift, -shift);
+        const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        f32x2 d[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) d[k] = f2_add(f2_from_bf16x2(w[k]), ns);
+        const f32x2 sum = f2_add(f2_add(f2_add(d[0], d[1]), f2_add(d[2], d[3])),
+                                 f2_add(f2_add(d[4], d[5]), f2_add(d[6], d[7])));
+        const f32x2 qa = f2_fma(d[0], d[0], f2_fma(d[1], d[1], f2_fma(d[2], d[2], f2_mul(d[3], d[3]))));
+        const f32x2 qb = f2_fma(d[4], d[4], f2_fma(d[5], d[5], f2_fma(d[6], d[6], f2_mul(d[7], d[7]))));
+        float t1 = f2_hsum(sum), t2 = f2_hsum(f2_add(qa, qb));
+#pragma unroll
+        for (int o = 2; o >= 1; o >>= 1) {
+            t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+            t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+        }
+        const float m1 = t1 * kInvC;
+        const float var = fmaxf(fmaf(-m1, m1, t2 * kInvC), 0.f);
+        const float rstd = rsqrtf(var + eps);
+        const float nm = -m1 * rstd;
+        const f32x2 r2 = f2_pack(rstd, rstd), n2 = f2_pack(nm, nm);
+        const bool zero = (zero_bits >> i) & 1u;
+        uint32_t o[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            o[k] = zero ? 0u : f2_to_bf16x2(f2_fma(f2_fma(d[k], r2, n2), gb[k], gb[8 + k]));
+        const uint4 y0 = make_uint4(o[0], o[1], o[2], o[3]), y1 = make_uint4(o[4], o[5], o[6], o[7]);
+        *reinterpret_cast<uint4*>(rowp + (odd ? off1 : off0)) = odd ? y1 : y0;
+        *reinterpret_cast<uint4*>(rowp + (odd ? off0 : off1)) = odd ? y0 : y1;
+    }
+}
+
+// gamma and beta of a lane's channels for ln_rows64_warp; 4-byte loads: the vectors may lie at any float address
+__device__ __forceinline__ void ln_load_affine_quad(f32x2 (&gb)[16], const float* gamma, const float* beta, int lane) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int ch = 8 * (lane & 3) + 32 * (k >> 2) + 2 * (k & 3);
+        gb[k] = f2_pack(__ldg(gamma + ch), __ldg(gamma + ch + 1));
+        gb[8 + k] = f2_pack(__ldg(beta + ch), __ldg(beta + ch + 1));
+    }
+}
+
 // gamma and beta of a lane's channels for ln_rows_warp, from global memory: lane chunk j = lane & 7 owns
 // channels [64 s + 8 j, 64 s + 8 j + 8) of every sub-tile s.
 template <int kSub>
@@ -819,6 +881,19 @@ __device__ __forceinline__ void ln_load_affine(f32x2 (&gb)[8 * kSub], const floa
         gb[4 * kSub + 4 * s + 0] = f2_pack(b0.x, b0.y); gb[4 * kSub + 4 * s + 1] = f2_pack(b0.z, b0.w);
         gb[4 * kSub + 4 * s + 2] = f2_pack(b1.x, b1.y); gb[4 * kSub + 4 * s + 3] = f2_pack(b1.z, b1.w);
     }
+}
+
+// The same with 4-byte loads, for kernels whose callers may pass LayerNorm vectors at any float address.
+template <int kSub>
+__device__ __forceinline__ void ln_load_affine_scalar(f32x2 (&gb)[8 * kSub], const float* gamma, const float* beta, int lane) {
+#pragma unroll
+    for (int s = 0; s < kSub; ++s)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int ch = 64 * s + 8 * (lane & 7) + 2 * k;
+            gb[4 * s + k] = f2_pack(__ldg(gamma + ch), __ldg(gamma + ch + 1));
+            gb[4 * kSub + 4 * s + k] = f2_pack(__ldg(beta + ch), __ldg(beta + ch + 1));
+        }
 }
 
 // Mean / rstd of one 128-channel row of a swizzled z tile (one pass, sums shifted by the row's

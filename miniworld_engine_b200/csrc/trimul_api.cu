@@ -401,30 +401,31 @@ int run_fast_tm1(const trimul_desc* d, const void* z, const uint8_t* mask, const
                         tmW[3], tmA, tmB, p);
 }
 
-// c = h = 64: left and right weights stacked into one UMMA operand (tm1_narrow_sm100.cuh)
+// h = 64, c = 64 or 128: left and right weights stacked into one UMMA operand (tm1_narrow_sm100.cuh)
 int run_narrow_tm1(const trimul_desc* d, const void* z, const uint8_t* mask, const trimul_weights* w,
                    const trimul_planes* a, const trimul_planes* b, cudaStream_t st, int32_t* status) {
     const bool inc = d->direction == TRIMUL_INCOMING;
+    const uint64_t C = (uint64_t)d->c;
     CUtensorMap tmZ, tmW[4], tmA, tmB;
     {
-        const uint64_t dims[4] = {kN1C, (uint64_t)d->N, (uint64_t)d->rows, (uint64_t)d->B};
-        const uint64_t strides[3] = {kN1C, (uint64_t)d->N * kN1C, (uint64_t)d->rows * d->N * kN1C};
+        const uint64_t dims[4] = {C, (uint64_t)d->N, (uint64_t)d->rows, (uint64_t)d->B};
+        const uint64_t strides[3] = {C, (uint64_t)d->N * C, (uint64_t)d->rows * d->N * C};
         const uint32_t box_out[4] = {64, 128, 1, 1};
         const uint32_t box_in[4] = {64, 1, 128, 1};
         if (!encode_bf16(&tmZ, z, 4, dims, strides, inc ? box_in : box_out, 128)) return TRIMUL_E_CUDA;
     }
     const void* ws[4] = {w->w_left, w->w_left_gate, w->w_right, w->w_right_gate};
     for (int m = 0; m < 4; ++m) {
-        const uint64_t dims[2] = {kN1C, kN1C};
-        const uint64_t strides[1] = {kN1C};
+        const uint64_t dims[2] = {C, kN1H};
+        const uint64_t strides[1] = {C};
         const uint32_t box[2] = {64, 64};
         if (!encode_bf16(&tmW[m], ws[m], 2, dims, strides, box, 128)) return TRIMUL_E_CUDA;
     }
-    const int planes = d->B * kN1C;
-    if (!encode_planes(&tmA, *a, planes, 64, 1, 64)) return TRIMUL_E_CUDA;
-    if (!encode_planes(&tmB, *b, planes, 64, 1, 64)) return TRIMUL_E_CUDA;
+    const int planes = d->B * kN1H;
+    if (!encode_planes(&tmA, *a, planes, 64, 1, 32)) return TRIMUL_E_CUDA;
+    if (!encode_planes(&tmB, *b, planes, 64, 1, 32)) return TRIMUL_E_CUDA;
     Tm1Params p = {};
-    p.B = d->B; p.c = kN1C;
+    p.B = d->B; p.c = d->c;
     p.n_fixed = inc ? d->N : d->rows;
     p.n_run = inc ? d->rows : d->N;
     p.tiles_per_fixed = (p.n_run + kT1P - 1) / kT1P;
@@ -441,9 +442,17 @@ int run_narrow_tm1(const trimul_desc* d, const void* z, const uint8_t* mask, con
     p.planes_per_dest = planes;
     p.status = status;
     const int grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
-    if (!ensure_smem(tm1_narrow_sm100_kernel, kN1SmemBytes)) return TRIMUL_E_CUDA;
-    return launch_stage(tm1_narrow_sm100_kernel, grid, kN1Threads, kN1SmemBytes, st, overlap_launches(d->flags), tmZ,
-                        tmW[0], tmW[1], tmW[2], tmW[3], tmA, tmB, p);
+    for (int k = 0; k < 2; ++k) {
+        p.step_q[k] = (k + 1) * grid / p.tiles_per_fixed;
+        p.step_r[k] = (k + 1) * grid % p.tiles_per_fixed;
+    }
+    auto launch = [&](auto kernel, int smem) {
+        if (!ensure_smem(kernel, smem)) return (int)TRIMUL_E_CUDA;
+        return launch_stage(kernel, grid, kN1Threads, smem, st, overlap_launches(d->flags), tmZ, tmW[0], tmW[1], tmW[2],
+                            tmW[3], tmA, tmB, p);
+    };
+    return d->c == 64 ? launch(tm1_narrow_sm100_kernel<1>, N1Layout<1>::kSmemBytes)
+                      : launch(tm1_narrow_sm100_kernel<2>, N1Layout<2>::kSmemBytes);
 }
 
 // c = h = 256: weights streamed through shared memory (tm1_wide_sm100.cuh)
@@ -836,7 +845,10 @@ int trimul_b200_tm1(const trimul_desc* desc, const void* z, const uint8_t* mask,
     if (tensor_core_path(desc) && desc->c_hidden == 128 && chunks_ok)
         return run_fast_tm1(desc, z, mask, w, a, b, st, status);
     if (wide_tensor_core_path(desc) && chunks_ok) return run_wide_tm1(desc, z, mask, w, a, b, st, status);
-    if (narrow_tensor_core_path(desc) && chunks_ok) return run_narrow_tm1(desc, z, mask, w, a, b, st, status);
+    // h = 64: the stacked-operand kernel (c = 128, bidirectional N = 320: 23 us a call,
+    // 159 on the warp-MMA kernel, which keeps the other widths)
+    if ((narrow_tensor_core_path(desc) || (tensor_core_path(desc) && desc->c_hidden == 64)) && chunks_ok)
+        return run_narrow_tm1(desc, z, mask, w, a, b, st, status);
     const void* mats[4] = {w->w_left, w->w_left_gate, w->w_right, w->w_right_gate};
     if (wmma_ok(desc, mats, 4)) return run_wmma_tm1(desc, z, mask, w, a, b, st);
     return run_plain_tm1<__nv_bfloat16>(desc, z, mask, w, a, b, st);
