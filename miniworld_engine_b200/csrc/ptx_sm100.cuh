@@ -896,10 +896,12 @@ __device__ __forceinline__ void ln_load_affine_scalar(f32x2 (&gb)[8 * kSub], con
         }
 }
 
-// Mean / rstd of one 128-channel row of a swizzled z tile (one pass, sums shifted by the row's
+// Mean / rstd of one row of 64 kSub channels of a swizzled z tile (one pass, sums shifted by the row's
 // first element so the variance does not cancel).  Returns rstd and t = -mean * rstd.
+template <int kSub = 2>
 __device__ __forceinline__ void row_stats(const uint8_t* tile, int sub_bytes, int row, float eps, float& rstd,
                                           float& t) {
+    constexpr float kInvC = 1.0f / (64.0f * kSub);
     const uint32_t swz = (uint32_t)(row & 7);
     const uint8_t* rowp = tile + row * 128;
     const uint32_t first = *reinterpret_cast<const uint32_t*>(rowp + (swz << 4));
@@ -908,7 +910,7 @@ __device__ __forceinline__ void row_stats(const uint8_t* tile, int sub_bytes, in
     f32x2 s1[4] = {0ull, 0ull, 0ull, 0ull}, s2[4] = {0ull, 0ull, 0ull, 0ull};
     // (short loop bodies on purpose: see the note on instruction-cache pressure at mbar_wait_slow)
 #pragma unroll 1
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < kSub; ++s) {
 #pragma unroll 4
         for (int j = 0; j < 8; ++j) {
             const uint4 v = *reinterpret_cast<const uint4*>(rowp + s * sub_bytes + ((((uint32_t)j) ^ swz) << 4));
@@ -921,9 +923,9 @@ __device__ __forceinline__ void row_stats(const uint8_t* tile, int sub_bytes, in
             }
         }
     }
-    const float m1 = f2_hsum(f2_add(f2_add(s1[0], s1[1]), f2_add(s1[2], s1[3]))) * (1.0f / 128.0f);
+    const float m1 = f2_hsum(f2_add(f2_add(s1[0], s1[1]), f2_add(s1[2], s1[3]))) * kInvC;
     const float q1 = f2_hsum(f2_add(f2_add(s2[0], s2[1]), f2_add(s2[2], s2[3])));
-    const float var = fmaxf(fmaf(-m1, m1, q1 * (1.0f / 128.0f)), 0.f);
+    const float var = fmaxf(fmaf(-m1, m1, q1 * kInvC), 0.f);
     rstd = rsqrtf(var + eps);
     t = -(shift + m1) * rstd;
 }

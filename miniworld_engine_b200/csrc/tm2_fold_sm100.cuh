@@ -1,4 +1,4 @@
-// Stage 3 of the block with BOTH LayerNorms folded into the projections, c = 128
+// Stage 3 of the block with BOTH LayerNorms folded into the projections, c = 64 or 128
 // (reference.py:76-83): out = sigmoid(Wg . LN_in(z)) * (Wo . LN_out(tri)) [+ z].
 //
 //   W . LN(x) = rstd * (W*gamma) . x  +  t * rowsum(W*gamma)  +  W . beta,      t = -mean * rstd
@@ -41,11 +41,15 @@
 // the block output before the residual (a template parameter: the inference instantiations carry
 // no trace of it).
 //
-// kKH = 2 is the last stage of the BIDIRECTIONAL block (bidirectional.py:150-156): tri has 256
+// kH = 256 is the last stage of the BIDIRECTIONAL block (bidirectional.py:150-156): tri has 256
 // channel planes per batch ([outgoing | incoming]), LayerNorm_out runs over all 256 and Wo is
 // [128, 256].  The tri tile then arrives as two 128-channel halves, each in one slot of the tri
 // ring (so a tile occupies the whole ring and the z ring is two deep: Wo takes 32 KB more); the
 // projection accumulates over both halves and the tri statistics are summed over both.
+// kH = 64 (c = 64, or a hidden width of half the pair width) has tri slots of 64 channels, four of them; with kC = 64
+// the z ring is six 16 KB tiles deep and the two epilogue groups share the tile's only 64-channel sub-tile.  Measured in
+// the step: c = 64, B = 2, N = 512 53 us instead of 74 with the LayerNorms in place, N = 1024 94 instead of 138;
+// c = 128, h = 64, N = 448 42 instead of 345 on the warp-MMA kernel.
 #pragma once
 
 #include "tm2_sm100.cuh"
@@ -55,17 +59,27 @@ namespace trimul {
 constexpr int kG2Threads = 640;
 constexpr int kG2EpiThreads = 256;      // warps 4..11, two groups of 128
 constexpr int kG2StatThreads = 128;     // each of the two statistics groups
-template <int kKH>
+// kC = channels of z and out (64, 128), kH = channels of tri (64, 128, 256)
+template <int kC, int kH>
 struct G2Layout {
-    static constexpr int kWBytes = (2 + 2 * kKH) * kT2SubTile;   // Wg: 2 K sub-tiles, Wo: 2 per 128 hidden channels
-    static constexpr int kZStages = kKH == 1 ? 3 : 2;
-    static constexpr int kOffZ = kWBytes;                        // z ring, 32 KB per stage
-    static constexpr int kOffT = kOffZ + kZStages * kT2XBytes;   // 2 x 32 KB tri ring; once a tile's tri data is dead the
+    static constexpr int kSlotCh = kH < 128 ? kH : 128;          // channel planes per tri slot
+    static constexpr int kSlots = kH / kSlotCh;                  // tri slots per tile
+    static constexpr int kWSub = kC * 128;                       // [kC output channels][64 k] of a weight matrix
+    static constexpr int kWBytes = (kC / 64 + kH / 64) * kWSub;  // Wg, then Wo
+    static constexpr int kZBytes = kC / 64 * kT2SubTile;         // z tile: 64-channel sub-tiles
+    static constexpr int kTSub = kSlotCh * 128;                  // [channels][64 positions] of a tri slot
+    static constexpr int kTBytes = 2 * kTSub;
+    static constexpr int kZStages = kC == 64 ? 6 : kH == 256 ? 2 : 3;
+    static constexpr int kTStages = kTBytes == 32768 ? 2 : 4;
+    static constexpr int kOffZ = kWBytes;
+    static constexpr int kOffT = kOffZ + kZStages * kZBytes;     // tri ring; once a tile's tri data is dead the
                                                                  // first 2 KB of its last slot hold [128 positions]
                                                                  // (r_in, t_in, r_out, t_out)
-    static constexpr int kOffConst = kOffT + 2 * kT2TBytes;      // [2 matrices][64 channel pairs] (s0, s1, b0, b1)
+    static constexpr int kOffConst = kOffT + kTStages * kTBytes; // [2 matrices][64 channel pairs] (s0, s1, b0, b1)
     static constexpr int kOffBars = kOffConst + 2048;
-    static constexpr int kSmemBytes = kOffBars + 256;
+    static constexpr int kSmemBytes = kOffBars + 384;
+    static_assert(kSmemBytes <= 232448, "folded stage 3 shared memory exceeds the 227 KB a CTA may use");
+    static_assert((10 + 4 * kZStages + 3 * kTStages) * 8 + 8 <= 384, "barrier block too small");
 };
 constexpr int kG2StatInBarrier = 2;
 constexpr int kG2StatOutBarrier = 3;
@@ -74,11 +88,11 @@ constexpr int kG2EpiBarrier = 4;        // 4: channels 0..63, 5: channels 64..12
 struct Tm2FoldParams {
     Tm2Params base;
     int residual_is_z;    // add the z tile to the result (the block's `pair + update` form)
-    const __nv_bfloat16* drop_scale;   // [B, 1, N, 128] row-broadcast multiplier of the block output
+    const __nv_bfloat16* drop_scale;   // [B, 1, N, c] row-broadcast multiplier of the block output
                                        // (module.py:332-337), applied before the residual; or null
 };
 
-template <bool kResidualIsZ, int kKH, bool kDropScale>
+template <bool kResidualIsZ, int kC, int kH, bool kDropScale>
 __global__ void __launch_bounds__(kG2Threads, 1)
 tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmWg,
                       const __grid_constant__ CUtensorMap tmWo, const __grid_constant__ CUtensorMap tmOut,
@@ -89,26 +103,27 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         if (threadIdx.x == 0) report_timeout(p.status, kStageIdTm2, 900);
         return;
     }
-    using L = G2Layout<kKH>;
-    constexpr int kG2ZStages = L::kZStages;
+    using L = G2Layout<kC, kH>;
+    constexpr int kG2ZStages = L::kZStages, kTS = L::kTStages, kSlots = L::kSlots, kSlotCh = L::kSlotCh;
+    constexpr int kCSub = kC / 64;              // 64-channel sub-tiles of z and out
     uint8_t* sW = smem;
     uint8_t* sZ = smem + L::kOffZ;
     uint8_t* sT = smem + L::kOffT;
     float4* sConst = reinterpret_cast<float4*>(smem + L::kOffConst);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBars);
-    uint64_t* w_full = bars;            // weights landed
-    uint64_t* w_ready = bars + 1;       // weights folded (256 arrivals)
-    uint64_t* z_full = bars + 2;        // [3] z tile landed
-    uint64_t* z_empty = bars + 5;       // [3] the store of the tile written over the z tile has read it (1 arrival)
-    uint64_t* box_ready = bars + 8;     // [3 stages][2 halves] result half written (4 arrivals)
-    uint64_t* t_full = bars + 14;       // [2] tri slot landed (a slot = 128 channel planes of a tile)
-    uint64_t* tri_dead = bars + 16;     // [2] the slot's UMMAs retired + its 128 statistics threads done reading
-    uint64_t* t_empty = bars + 18;      // [2] the epilogue has taken the statistics out of the slot (8 arrivals)
-    uint64_t* acc_full = bars + 20;     // [2]
-    uint64_t* acc_empty = bars + 22;    // [2] (8 arrivals)
-    uint64_t* stat_in = bars + 24;      // [2] z statistics written into the tri buffer (128 arrivals)
-    uint64_t* stat_out = bars + 26;     // [2] tri statistics written (128 arrivals)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
+    uint64_t* w_full = bars;                    // weights landed
+    uint64_t* w_ready = bars + 1;               // weights folded (256 arrivals)
+    uint64_t* z_full = bars + 2;                // [z stages] z tile landed
+    uint64_t* z_empty = z_full + kG2ZStages;    // [z stages] the store of the tile written over the z tile has read it (1 arrival)
+    uint64_t* box_ready = z_empty + kG2ZStages; // [z stages][2 halves] result half written (4 arrivals)
+    uint64_t* t_full = box_ready + 2 * kG2ZStages;   // [tri stages] tri slot landed (a slot = kSlotCh channel planes of a tile)
+    uint64_t* tri_dead = t_full + kTS;          // [tri stages] the slot's UMMAs retired + its 128 statistics threads done reading
+    uint64_t* t_empty = tri_dead + kTS;         // [tri stages] the epilogue has taken the statistics out of the slot (8 arrivals)
+    uint64_t* acc_full = t_empty + kTS;         // [2]
+    uint64_t* acc_empty = acc_full + 2;         // [2] (8 arrivals)
+    uint64_t* stat_in = acc_empty + 2;          // [2] z statistics written into the tri buffer (128 arrivals)
+    uint64_t* stat_out = stat_in + 2;           // [2] tri statistics written (128 arrivals)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stat_out + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
@@ -123,10 +138,12 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             mbar_init(&box_ready[2 * s], 4);
             mbar_init(&box_ready[2 * s + 1], 4);
         }
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < kTS; ++s) {
             mbar_init(&t_full[s], 1);
             mbar_init(&tri_dead[s], 1 + kG2StatThreads);
             mbar_init(&t_empty[s], 8);
+        }
+        for (int s = 0; s < 2; ++s) {
             mbar_init(&acc_full[s], 1);
             mbar_init(&acc_empty[s], 8);
             mbar_init(&stat_in[s], kG2StatThreads);
@@ -154,8 +171,8 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
             mbar_arrive_expect_tx(w_full, L::kWBytes);
-            for (int kh = 0; kh < 2; ++kh) tma_load_2d(sW + kh * kT2SubTile, &tmWg, w_full, kh * 64, 0);
-            for (int kh = 0; kh < 2 * kKH; ++kh) tma_load_2d(sW + (2 + kh) * kT2SubTile, &tmWo, w_full, kh * 64, 0);
+            for (int kh = 0; kh < kCSub; ++kh) tma_load_2d(sW + kh * L::kWSub, &tmWg, w_full, kh * 64, 0);
+            for (int kh = 0; kh < kH / 64; ++kh) tma_load_2d(sW + (kCSub + kh) * L::kWSub, &tmWo, w_full, kh * 64, 0);
             uint32_t it = 0;
             for (int tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
                 const int zs = it % kG2ZStages;
@@ -165,40 +182,39 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                 const int r = br % p.rows;
                 const int b = br / p.rows;
                 bool okp = true;
-                for (int h = 0; h < kKH; ++h) {
-                    // tri slot of this 128-channel half: slots are used round-robin, use n = u >> 1
-                    const uint32_t u = it * kKH + h;
-                    const int ts = u & 1;
-                    const uint32_t tph = (u >> 1) & 1u;
+                for (int h = 0; h < kSlots; ++h) {
+                    // tri slot of this part of the channels: slots are used round-robin, use n = u / kTS
+                    const uint32_t u = it * kSlots + h;
+                    const int ts = u % kTS;
+                    const uint32_t tph = (u / kTS) & 1u;
                     // a tile's LAST slot carries the statistics and is released by the epilogue; any
                     // other slot is free as soon as its readers are done (so the next tile's first half
                     // streams in while this tile's last half is still being worked on)
-                    uint64_t* freed = h == kKH - 1 ? &t_empty[ts] : &tri_dead[ts];
+                    uint64_t* freed = h == kSlots - 1 ? &t_empty[ts] : &tri_dead[ts];
                     if (!mbar_wait<true>(freed, tph ^ 1u, abort_flag, p.status, kStageIdTm2, 100 + ts)) {
                         okp = false;
                         break;
                     }
-                    // tri planes viewed as (column, row, plane, chunk): 64 columns x 128 planes per box
-                    mbar_arrive_expect_tx(&t_full[ts], kT2TBytes);
-                    uint8_t* dt = sT + ts * kT2TBytes;
-                    tma_load_4d(dt, &tmTri, &t_full[ts], j0, r, (b * kKH + h) * kT2C, 0);
-                    tma_load_4d(dt + kT2SubTile, &tmTri, &t_full[ts], j0 + 64, r, (b * kKH + h) * kT2C, 0);
+                    // tri planes viewed as (column, row, plane, chunk): 64 columns x kSlotCh planes per box
+                    mbar_arrive_expect_tx(&t_full[ts], L::kTBytes);
+                    uint8_t* dt = sT + ts * L::kTBytes;
+                    tma_load_4d(dt, &tmTri, &t_full[ts], j0, r, (b * kSlots + h) * kSlotCh, 0);
+                    tma_load_4d(dt + L::kTSub, &tmTri, &t_full[ts], j0 + 64, r, (b * kSlots + h) * kSlotCh, 0);
                 }
                 if (!okp) break;
                 if (!mbar_wait<true>(&z_empty[zs], zph ^ 1u, abort_flag, p.status, kStageIdTm2, 110 + zs)) break;
                 TRIMUL_STAMP(0, it, 0);
-                mbar_arrive_expect_tx(&z_full[zs], kT2XBytes);
-                uint8_t* dz = sZ + zs * kT2XBytes;
-                tma_load_4d(dz, &tmZ, &z_full[zs], 0, j0, r, b);
-                tma_load_4d(dz + kT2SubTile, &tmZ, &z_full[zs], 64, j0, r, b);
+                mbar_arrive_expect_tx(&z_full[zs], L::kZBytes);
+                uint8_t* dz = sZ + zs * L::kZBytes;
+                for (int ks = 0; ks < kCSub; ++ks) tma_load_4d(dz + ks * kT2SubTile, &tmZ, &z_full[zs], ks * 64, j0, r, b);
             }
         }
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------------ UMMA issuer
         if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(kT2P, kT2C);
-            constexpr uint32_t idesc_mn = umma_idesc_bf16(kT2P, kT2C, 1, 0);   // A (tri) is MN-major
+            constexpr uint32_t idesc = umma_idesc_bf16(kT2P, kC);
+            constexpr uint32_t idesc_mn = umma_idesc_bf16(kT2P, kC, 1, 0);   // A (tri) is MN-major
             bool ok = mbar_wait<true>(w_ready, 0, abort_flag, p.status, kStageIdTm2, 200);
             tcgen05_fence_after();
             uint32_t it = 0;
@@ -208,26 +224,26 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                 // accumulator pair `s` was last used by tile it-2
                 if (!mbar_wait<true>(&acc_empty[s], ph ^ 1u, abort_flag, p.status, kStageIdTm2, 210 + s)) break;
                 const uint32_t wg = smem_u32(sW);
-                const uint32_t wo = wg + 2 * kT2SubTile;
+                const uint32_t wo = wg + kCSub * L::kWSub;
                 const uint32_t d_g = tmem_base + s * 256;
                 const uint32_t d_p = d_g + 128;
-                for (int h = 0; ok && h < kKH; ++h) {
-                    const uint32_t u = it * kKH + h;
-                    const int tsl = u & 1;
-                    if (!mbar_wait<true>(&t_full[tsl], (u >> 1) & 1u, abort_flag, p.status, kStageIdTm2, 230 + tsl)) {
+                for (int h = 0; ok && h < kSlots; ++h) {
+                    const uint32_t u = it * kSlots + h;
+                    const int tsl = u % kTS;
+                    if (!mbar_wait<true>(&t_full[tsl], (u / kTS) & 1u, abort_flag, p.status, kStageIdTm2, 230 + tsl)) {
                         ok = false;
                         break;
                     }
                     tcgen05_fence_after();
                     TRIMUL_STAMP(1, it, 0);
-                    const uint32_t ts = smem_u32(sT + tsl * kT2TBytes);
-                    const uint32_t woh = wo + h * 2 * kT2SubTile;       // Wo columns of this half
+                    const uint32_t ts = smem_u32(sT + tsl * L::kTBytes);
+                    const uint32_t woh = wo + h * (kSlotCh / 64) * L::kWSub;       // Wo columns of this slot
 #pragma unroll 2
-                    for (int kk = 0; kk < kT2C / 16; ++kk) {
+                    for (int kk = 0; kk < kSlotCh / 16; ++kk) {
                         // tri slot: rows are channels (K), 128 bytes = 64 positions per row, the second
                         // 64 positions one sub-tile further; a K step of 16 is two 8-row groups = 2048 B
-                        umma_bf16_ss(d_p, umma_smem_desc_mn_sw128(ts + kk * 2048, kT2SubTile, 1024),
-                                     umma_smem_desc_sw128(woh + (kk >> 2) * kT2SubTile) + (kk & 3) * kDescKStep,
+                        umma_bf16_ss(d_p, umma_smem_desc_mn_sw128(ts + kk * 2048, L::kTSub, 1024),
+                                     umma_smem_desc_sw128(woh + (kk >> 2) * L::kWSub) + (kk & 3) * kDescKStep,
                                      idesc_mn, (kk | h) != 0);
                     }
                     umma_commit(&tri_dead[tsl]);
@@ -237,13 +253,12 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                 if (!mbar_wait<true>(&z_full[zs], (it / kG2ZStages) & 1u, abort_flag, p.status, kStageIdTm2, 220 + zs)) break;
                 tcgen05_fence_after();
                 TRIMUL_STAMP(1, it, 1);
-                const uint32_t xs = smem_u32(sZ + zs * kT2XBytes);
+                const uint32_t xs = smem_u32(sZ + zs * L::kZBytes);
 #pragma unroll 2
-                for (int kk = 0; kk < kT2C / 16; ++kk) {
-                    const uint32_t sub = (kk >> 2) * kT2SubTile;
+                for (int kk = 0; kk < kC / 16; ++kk) {
                     const uint64_t kofs = (kk & 3) * kDescKStep;
-                    umma_bf16_ss(d_g, umma_smem_desc_sw128(xs + sub) + kofs, umma_smem_desc_sw128(wg + sub) + kofs,
-                                 idesc, kk != 0);
+                    umma_bf16_ss(d_g, umma_smem_desc_sw128(xs + (kk >> 2) * kT2SubTile) + kofs,
+                                 umma_smem_desc_sw128(wg + (kk >> 2) * L::kWSub) + kofs, idesc, kk != 0);
                 }
                 umma_commit(&acc_full[s]);
                 TRIMUL_STAMP(1, it, 2);
@@ -261,12 +276,15 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                 const int br = tile / p.tiles_per_row;
                 const int r = br % p.rows;
                 const int b = br / p.rows;
-                const uint8_t* src = sZ + s * kT2XBytes;
+                const uint8_t* src = sZ + s * L::kZBytes;
                 if (!mbar_wait<true>(&box_ready[2 * s], ph, abort_flag, p.status, kStageIdTm2, 600 + s)) break;
-                tma_store_4d(&tmOut, src, 0, j0, r, b);
-                tma_store_commit();
+                if (kC == 128) {
+                    tma_store_4d(&tmOut, src, 0, j0, r, b);
+                    tma_store_commit();
+                }
                 if (!mbar_wait<true>(&box_ready[2 * s + 1], ph, abort_flag, p.status, kStageIdTm2, 610 + s)) break;
-                tma_store_4d(&tmOut, src + kT2SubTile, 64, j0, r, b);
+                if (kC == 128) tma_store_4d(&tmOut, src + kT2SubTile, 64, j0, r, b);
+                else tma_store_4d(&tmOut, src, 0, j0, r, b);
                 tma_store_commit();
                 tma_store_wait_read<0>();
                 TRIMUL_STAMP(2, it, 0);
@@ -280,7 +298,7 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     } else if (warp < 12) {
         // ------------------------------------------------------------------ epilogue
         const int e = threadIdx.x - 128;               // 0..255
-        const int grp = e >> 7;                        // channel half: 0 -> channels 0..63, 1 -> 64..127
+        const int grp = e >> 7;                        // half of the output channels
         const int q = warp & 3;
         const int row = q * 32 + lane;                 // position inside the tile == TMEM lane
         const bool leader = (e & 127) == 0;
@@ -290,12 +308,14 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         bool run = mbar_wait<true>(w_full, 0, abort_flag, p.status, kStageIdTm2, 150);
         if (run) {
             const int m = e >> 7, n = e & 127;
-            float s_, b_;
-            fold_row_smem(sW + m * 2 * kT2SubTile, kT2SubTile, n, m == 0 ? p.gamma_in : p.gamma_out,
-                          m == 0 ? p.beta_in : p.beta_out, m == 0 ? 2 : 2 * kKH, s_, b_);
-            float* c = reinterpret_cast<float*>(&sConst[m * 64 + (n >> 1)]);
-            c[n & 1] = s_;
-            c[2 + (n & 1)] = b_;
+            if (n < kC) {
+                float s_, b_;
+                fold_row_smem(sW + m * kCSub * L::kWSub, L::kWSub, n, m == 0 ? p.gamma_in : p.gamma_out,
+                              m == 0 ? p.beta_in : p.beta_out, m == 0 ? kCSub : kH / 64, s_, b_);
+                float* c = reinterpret_cast<float*>(&sConst[m * 64 + (n >> 1)]);
+                c[n & 1] = s_;
+                c[2 + (n & 1)] = b_;
+            }
             fence_proxy_async_smem();      // folded weights -> visible to the UMMA (async proxy)
         }
         mbar_arrive(w_ready);
@@ -305,7 +325,7 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         run = named_barrier_all(bar_id, 128, run);
 
         const uint32_t lane_bits = (uint32_t)(q * 32) << 16;
-        const ulonglong2* cG = reinterpret_cast<const ulonglong2*>(sConst) + grp * 32;
+        const ulonglong2* cG = reinterpret_cast<const ulonglong2*>(sConst) + grp * (kC / 4);
         const ulonglong2* cO = cG + 64;
         uint32_t it = 0;
         for (int tile = blockIdx.x; run && tile < p.total_tiles; tile += gridDim.x, ++it) {
@@ -321,26 +341,28 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             if (!named_barrier_all(bar_id, 128, ok)) break;
             tcgen05_fence_after();
             if (e == 0) TRIMUL_STAMP(4, it, 0);
-            const int slot0 = (it * kKH + kKH - 1) & 1;     // the tile's last tri slot carries its statistics
-            const float4 st = reinterpret_cast<const float4*>(sT + slot0 * kT2TBytes)[row];
+            const int slot0 = (it * kSlots + kSlots - 1) % kTS;     // the tile's last tri slot carries its statistics
+            const float4 st = reinterpret_cast<const float4*>(sT + slot0 * L::kTBytes)[row];
             __syncwarp();
             if (lane == 0) mbar_arrive(&t_empty[slot0]);    // this warp has its statistics: the slot may be refilled
             const f32x2 rin = f2_pack(st.x, st.x), tin = f2_pack(st.y, st.y);
             const f32x2 rout = f2_pack(st.z, st.z), tout = f2_pack(st.w, st.w);
-            const uint32_t t_g = tmem_base + s * 256 + grp * 64 + lane_bits;     // gate; proj 128 columns on
-            uint8_t* tile_row = sZ + zs * kT2XBytes + grp * kT2SubTile + row * 128;
-            // this position's 64 drop-scale values (it is column j0 + row of z row r, any r)
+            const uint32_t t_g = tmem_base + s * 256 + grp * (kC / 2) + lane_bits;     // gate; proj 128 columns on
+            // kC = 128: the group's half is a sub-tile; kC = 64: the second four 16-byte chunks of the only one
+            uint8_t* tile_row = sZ + zs * L::kZBytes + (kC == 128 ? grp * kT2SubTile : 0) + row * 128;
+            const int chunk0 = kC == 128 ? 0 : grp * 4;
+            // this position's drop-scale values (it is column j0 + row of z row r, any r)
             const __nv_bfloat16* ds_row = nullptr;
             if (kDropScale) {
                 const int j0 = (tile % p.tiles_per_row) * kT2P;
                 const int b = (tile / p.tiles_per_row) / p.rows;
-                if (j0 + row < p.N) ds_row = fp.drop_scale + ((size_t)b * p.N + j0 + row) * kT2C + grp * 64;
+                if (j0 + row < p.N) ds_row = fp.drop_scale + ((size_t)b * p.N + j0 + row) * kC + grp * (kC / 2);
             }
             // 8 output channels (one 16-byte chunk) at a time; the TMEM loads of the next 8 are in
             // flight while the current 8 get their statistics, are gated, rounded and written over the
             // z tile.  The loop stays rolled to keep the code small.
             auto emit8 = [&](int c8, const uint32_t (&rg)[8], const uint32_t (&rp)[8]) {
-                uint4* dst = reinterpret_cast<uint4*>(tile_row + ((c8 ^ (row & 7)) << 4));
+                uint4* dst = reinterpret_cast<uint4*>(tile_row + (((chunk0 + c8) ^ (row & 7)) << 4));
                 uint32_t res[4] = {0u, 0u, 0u, 0u};
                 if (kResidualIsZ) {
                     const uint4 rv = *dst;
@@ -373,13 +395,13 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             tmem_ld_32x8(t_g, rgA);
             tmem_ld_32x8(t_g + 128, rpA);
 #pragma unroll 1
-            for (int c8 = 0; c8 < 8; c8 += 2) {
+            for (int c8 = 0; c8 < kC / 16; c8 += 2) {
                 tmem_ld_wait();
                 tmem_ld_32x8(t_g + (c8 + 1) * 8, rgB);
                 tmem_ld_32x8(t_g + 128 + (c8 + 1) * 8, rpB);
                 emit8(c8, rgA, rpA);
                 tmem_ld_wait();
-                if (c8 + 2 < 8) {
+                if (c8 + 2 < kC / 16) {
                     tmem_ld_32x8(t_g + (c8 + 2) * 8, rgA);
                     tmem_ld_32x8(t_g + 128 + (c8 + 2) * 8, rpA);
                 } else {
@@ -407,14 +429,14 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                 break;
             if (pos == 0) TRIMUL_STAMP(3, it, 0);
             float rstd, t;
-            row_stats(sZ + zs * kT2XBytes, kT2SubTile, pos, p.eps_in, rstd, t);
+            row_stats<kCSub>(sZ + zs * L::kZBytes, kT2SubTile, pos, p.eps_in, rstd, t);
             // the statistics go into the tile's last tri slot once nothing reads the tri data there any more
-            const uint32_t u0 = it * kKH + kKH - 1;
-            const int slot0 = u0 & 1;
-            if (!group_wait<true>(&tri_dead[slot0], (u0 >> 1) & 1u, pos == 0, kG2StatInBarrier, kG2StatThreads,
+            const uint32_t u0 = it * kSlots + kSlots - 1;
+            const int slot0 = u0 % kTS;
+            if (!group_wait<true>(&tri_dead[slot0], (u0 / kTS) & 1u, pos == 0, kG2StatInBarrier, kG2StatThreads,
                                   abort_flag, p.status, kStageIdTm2, 310 + slot0))
                 break;
-            *reinterpret_cast<float2*>(reinterpret_cast<float4*>(sT + slot0 * kT2TBytes) + pos) = make_float2(rstd, t);
+            *reinterpret_cast<float2*>(reinterpret_cast<float4*>(sT + slot0 * L::kTBytes) + pos) = make_float2(rstd, t);
             mbar_arrive(&stat_in[s]);
             if (pos == 0) TRIMUL_STAMP(3, it, 1);
         }
@@ -422,15 +444,15 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         // ------------------------------------------------------------------ statistics of the tri tile
         // The tile is [128 channel rows][128 positions] as two 64-position sub-tiles, 16-byte chunk c
         // of row r stored at chunk c ^ (r & 7).  Thread (tw, ql, rs): position chunk cq = 4 tw + ql
-        // (positions 8 cq .. 8 cq + 7), channel rows rs, rs + 8, ..., rs + 120; all its rows have
+        // (positions 8 cq .. 8 cq + 7), channel rows rs, rs + 8, ...; all its rows have
         // r & 7 == rs, so its 16 bytes sit at the same offset in every row.
         const int tid = threadIdx.x - 512;             // 0..127
         const int tw = tid >> 5;
         const int ql = lane >> 3;
         const int rs = lane & 7;
         const int cq = 4 * tw + ql;
-        const uint32_t col_off = (uint32_t)(cq >> 3) * kT2SubTile + ((((uint32_t)cq & 7u) ^ (uint32_t)rs) << 4);
-        const float inv_c = 1.0f / (float)(kT2C * kKH);
+        const uint32_t col_off = (uint32_t)(cq >> 3) * L::kTSub + ((((uint32_t)cq & 7u) ^ (uint32_t)rs) << 4);
+        const float inv_c = 1.0f / (float)kH;
         uint32_t it = 0;
         bool alive = true;
         for (int tile = blockIdx.x; alive && tile < p.total_tiles; tile += gridDim.x, ++it) {
@@ -438,16 +460,16 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             uint32_t sh[4] = {0u, 0u, 0u, 0u};
             f32x2 nsh[4] = {0ull, 0ull, 0ull, 0ull}, a[4] = {0ull, 0ull, 0ull, 0ull}, qq[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll 1
-            for (int h = 0; h < kKH; ++h) {           // the tile's 128-channel halves, one tri slot each
-                const uint32_t u = it * kKH + h;
-                const int ts = u & 1;
-                if (!group_wait<true>(&t_full[ts], (u >> 1) & 1u, tid == 0, kG2StatOutBarrier, kG2StatThreads, abort_flag,
+            for (int h = 0; h < kSlots; ++h) {        // the tile's tri slots
+                const uint32_t u = it * kSlots + h;
+                const int ts = u % kTS;
+                if (!group_wait<true>(&t_full[ts], (u / kTS) & 1u, tid == 0, kG2StatOutBarrier, kG2StatThreads, abort_flag,
                                       p.status, kStageIdTm2, 500 + ts)) {
                     alive = false;
                     break;
                 }
                 if (tid == 0) TRIMUL_STAMP(5, it, 0);
-                const uint8_t* base = sT + ts * kT2TBytes + col_off + rs * 128;
+                const uint8_t* base = sT + ts * L::kTBytes + col_off + rs * 128;
                 if (h == 0) {
                     // common shift of each position: its channel 0 (row 0, held by the rs == 0 lane)
                     const uint4 v0 = *reinterpret_cast<const uint4*>(base);
@@ -459,7 +481,7 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                     for (int w = 0; w < 4; ++w) nsh[w] = f2_pack(-bf16_lo(sh[w]), -bf16_hi(sh[w]));
                 }
 #pragma unroll 4
-                for (int m = 0; m < 16; ++m) {
+                for (int m = 0; m < kSlotCh / 8; ++m) {
                     const uint4 v = *reinterpret_cast<const uint4*>(base + m * 1024);
                     const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -497,13 +519,13 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             const float rstd = rsqrtf(fmaxf(fmaf(-m1, m1, s2[0] * inv_c), 0.f) + p.eps_out);
             const float t = -(shift + m1) * rstd;
             // the statistics go into the tile's last tri slot once nothing reads the tri data there any more
-            const uint32_t u0 = it * kKH + kKH - 1;
-            const int slot0 = u0 & 1;
-            if (!group_wait<true>(&tri_dead[slot0], (u0 >> 1) & 1u, tid == 0, kG2StatOutBarrier, kG2StatThreads, abort_flag,
+            const uint32_t u0 = it * kSlots + kSlots - 1;
+            const int slot0 = u0 % kTS;
+            if (!group_wait<true>(&tri_dead[slot0], (u0 / kTS) & 1u, tid == 0, kG2StatOutBarrier, kG2StatThreads, abort_flag,
                                   p.status, kStageIdTm2, 510 + slot0))
                 break;
             // position 8 cq + rs == tid
-            *(reinterpret_cast<float2*>(reinterpret_cast<float4*>(sT + slot0 * kT2TBytes) + tid) + 1) = make_float2(rstd, t);
+            *(reinterpret_cast<float2*>(reinterpret_cast<float4*>(sT + slot0 * L::kTBytes) + tid) + 1) = make_float2(rstd, t);
             mbar_arrive(&stat_out[s]);
             if (tid == 0) TRIMUL_STAMP(5, it, 1);
         }

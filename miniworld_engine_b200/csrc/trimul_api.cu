@@ -633,8 +633,60 @@ int run_wmma_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri, 
     return launch_status();
 }
 
-int run_fast_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri, const trimul_weights* w, void* out,
+Tm2Params tm2_params(const trimul_desc* d, const trimul_weights* w, const void* residual, int32_t* status) {
+    Tm2Params p = {};
+    p.B = d->B; p.rows = d->rows; p.N = d->N;
+    p.tiles_per_row = (d->N + kT2P - 1) / kT2P;
+    p.total_tiles = d->B * d->rows * p.tiles_per_row;
+    p.gamma_in = w->ln_in_weight; p.beta_in = w->ln_in_bias;
+    p.gamma_out = w->ln_out_weight; p.beta_out = w->ln_out_bias;
+    p.eps_in = d->eps_in; p.eps_out = d->eps_out;
+    p.has_residual = residual != nullptr;
+    p.status = status;
+    return p;
+}
+
+// both LayerNorms folded into the weights, result written in place over the z tile (tm2_fold_sm100.cuh);
+// residual: null or z itself (another tensor needs a tile buffer this kernel does not have)
+template <int kC, int kH>
+int run_fold_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri, const trimul_weights* w, void* out,
                  const void* residual, cudaStream_t st, int32_t* status) {
+    using L = G2Layout<kC, kH>;
+    if ((int64_t)d->B * d->rows * ((d->N + kT2P - 1) / kT2P) > 0x7fffffff) return TRIMUL_E_UNSUPPORTED;
+    CUtensorMap tmZ, tmWg, tmWo, tmOut, tmTri;
+    const uint64_t dims[4] = {kC, (uint64_t)d->N, (uint64_t)d->rows, (uint64_t)d->B};
+    const uint64_t strides[3] = {kC, (uint64_t)d->N * kC, (uint64_t)d->rows * d->N * kC};
+    const uint32_t box[4] = {64, 128, 1, 1};
+    if (!encode_bf16(&tmZ, z, 4, dims, strides, box, 128)) return TRIMUL_E_CUDA;
+    if (!encode_bf16(&tmOut, out, 4, dims, strides, box, 128)) return TRIMUL_E_CUDA;
+    const uint64_t wdims[2] = {kC, kC}, wstrides[1] = {kC};
+    const uint64_t wodims[2] = {kH, kC}, wostrides[1] = {kH};
+    const uint32_t wbox[2] = {64, kC};
+    if (!encode_bf16(&tmWg, w->w_gate, 2, wdims, wstrides, wbox, 128)) return TRIMUL_E_CUDA;
+    if (!encode_bf16(&tmWo, w->w_out, 2, wodims, wostrides, wbox, 128)) return TRIMUL_E_CUDA;
+    if (!encode_planes(&tmTri, *tri, d->B * kH, 64, 1, L::kSlotCh)) return TRIMUL_E_CUDA;
+    Tm2FoldParams fp;
+    fp.base = tm2_params(d, w, residual, status);
+    fp.residual_is_z = residual != nullptr;
+    fp.drop_scale = static_cast<const __nv_bfloat16*>(desc_drop_scale(d));
+    const int grid = fp.base.total_tiles < sm_count() ? fp.base.total_tiles : sm_count();
+    auto launch = [&](auto kernel) {
+        if (!ensure_smem(kernel, L::kSmemBytes)) return (int)TRIMUL_E_CUDA;
+        return launch_stage(kernel, grid, kG2Threads, L::kSmemBytes, st, overlap_launches(d->flags), tmZ, tmWg, tmWo, tmOut,
+                            tmTri, fp);
+    };
+    if (fp.drop_scale != nullptr)
+        return residual != nullptr ? launch(tm2_fold_sm100_kernel<true, kC, kH, true>)
+                                   : launch(tm2_fold_sm100_kernel<false, kC, kH, true>);
+    return residual != nullptr ? launch(tm2_fold_sm100_kernel<true, kC, kH, false>)
+                               : launch(tm2_fold_sm100_kernel<false, kC, kH, false>);
+}
+
+// c = h = 128 with a residual that is not z (or on request): both LayerNorms in place (tm2_sm100.cuh)
+int run_inplace_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri, const trimul_weights* w, void* out,
+                    const void* residual, cudaStream_t st, int32_t* status) {
+    if (desc_drop_scale(d) != nullptr) return TRIMUL_E_UNSUPPORTED;      // no drop-scale operand
+    if ((int64_t)d->B * d->rows * ((d->N + kT2P - 1) / kT2P) > 0x7fffffff) return TRIMUL_E_UNSUPPORTED;
     CUtensorMap tmZ, tmWg, tmWo, tmOut, tmRes, tmTri;
     const uint64_t dims[4] = {128, (uint64_t)d->N, (uint64_t)d->rows, (uint64_t)d->B};
     const uint64_t strides[3] = {128, (uint64_t)d->N * 128, (uint64_t)d->rows * d->N * 128};
@@ -642,57 +694,13 @@ int run_fast_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri, 
     if (!encode_bf16(&tmZ, z, 4, dims, strides, box, 128)) return TRIMUL_E_CUDA;
     if (!encode_bf16(&tmOut, out, 4, dims, strides, box, 128)) return TRIMUL_E_CUDA;
     if (!encode_bf16(&tmRes, residual ? residual : z, 4, dims, strides, box, 128)) return TRIMUL_E_CUDA;
-    const int kh = d->c_hidden / 128;          // 1, or 2 for the bidirectional block's last stage
-    const uint64_t wdims[2] = {128, 128};
-    const uint64_t wstrides[1] = {128};
-    const uint64_t wodims[2] = {(uint64_t)d->c_hidden, 128};
-    const uint64_t wostrides[1] = {(uint64_t)d->c_hidden};
+    const uint64_t wdims[2] = {128, 128}, wstrides[1] = {128};
     const uint32_t wbox[2] = {64, 128};
     if (!encode_bf16(&tmWg, w->w_gate, 2, wdims, wstrides, wbox, 128)) return TRIMUL_E_CUDA;
-    if (!encode_bf16(&tmWo, w->w_out, 2, wodims, wostrides, wbox, 128)) return TRIMUL_E_CUDA;
-    Tm2Params p;
-    p.B = d->B; p.rows = d->rows; p.N = d->N;
-    p.tiles_per_row = (d->N + kT2P - 1) / kT2P;
-    const int64_t total = (int64_t)d->B * d->rows * p.tiles_per_row;
-    if (total > 0x7fffffff) return TRIMUL_E_UNSUPPORTED;
-    p.total_tiles = (int)total;
-    if (!encode_planes(&tmTri, *tri, d->B * d->c_hidden, 64, 1, 128)) return TRIMUL_E_CUDA;
-    p.gamma_in = w->ln_in_weight; p.beta_in = w->ln_in_bias;
-    p.gamma_out = w->ln_out_weight; p.beta_out = w->ln_out_bias;
-    p.eps_in = d->eps_in; p.eps_out = d->eps_out;
-    p.has_residual = residual != nullptr;
-    p.status = status;
+    if (!encode_bf16(&tmWo, w->w_out, 2, wdims, wstrides, wbox, 128)) return TRIMUL_E_CUDA;
+    if (!encode_planes(&tmTri, *tri, d->B * 128, 64, 1, 128)) return TRIMUL_E_CUDA;
+    const Tm2Params p = tm2_params(d, w, residual, status);
     const int grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
-    if ((d->flags & TRIMUL_FLAG_INPLACE_NORM_STAGE3) == 0 && (residual == nullptr || residual == z)) {
-        // default: both LayerNorms folded into the weights, result written in place over the z tile
-        // (a residual other than z itself needs a tile buffer this kernel does not have)
-        Tm2FoldParams fp;
-        fp.base = p;
-        fp.residual_is_z = residual != nullptr;
-        fp.drop_scale = static_cast<const __nv_bfloat16*>(desc_drop_scale(d));
-#define TRIMUL_LAUNCH_TM2_FOLD(RES, KH, DS)                                                                       \
-    do {                                                                                                           \
-        if (!ensure_smem(tm2_fold_sm100_kernel<RES, KH, DS>, G2Layout<KH>::kSmemBytes)) return TRIMUL_E_CUDA;       \
-        return launch_stage(tm2_fold_sm100_kernel<RES, KH, DS>, grid, kG2Threads, G2Layout<KH>::kSmemBytes, st,     \
-                            overlap_launches(d->flags), tmZ, tmWg, tmWo, tmOut, tmTri, fp);                        \
-    } while (0)
-#define TRIMUL_LAUNCH_TM2_FOLD_RK(RES, KH)                  \
-    do {                                                    \
-        if (fp.drop_scale != nullptr) TRIMUL_LAUNCH_TM2_FOLD(RES, KH, true); \
-        else TRIMUL_LAUNCH_TM2_FOLD(RES, KH, false);        \
-    } while (0)
-        if (kh == 2) {
-            if (residual != nullptr) TRIMUL_LAUNCH_TM2_FOLD_RK(true, 2);
-            else TRIMUL_LAUNCH_TM2_FOLD_RK(false, 2);
-        } else {
-            if (residual != nullptr) TRIMUL_LAUNCH_TM2_FOLD_RK(true, 1);
-            else TRIMUL_LAUNCH_TM2_FOLD_RK(false, 1);
-        }
-#undef TRIMUL_LAUNCH_TM2_FOLD_RK
-#undef TRIMUL_LAUNCH_TM2_FOLD
-    }
-    if (kh != 1) return TRIMUL_E_UNSUPPORTED;      // the in-place variant below is 128 hidden channels only
-    if (desc_drop_scale(d) != nullptr) return TRIMUL_E_UNSUPPORTED;   // ... and has no drop-scale operand
     if (!ensure_smem(tm2_sm100_kernel, kT2SmemBytes)) return TRIMUL_E_CUDA;
     tm2_sm100_kernel<<<grid, kT2Threads, kT2SmemBytes, st>>>(tmZ, tmWg, tmWo, tmOut, tmRes, tmTri, p);
     return launch_status();
@@ -955,11 +963,21 @@ int trimul_b200_tm2(const trimul_desc* desc, const void* z, const trimul_planes*
     if (desc->dtype == TRIMUL_DTYPE_FP32) return run_plain_tm2<float>(desc, z, tri, w, out, residual, st);
     const bool plain_layout = tri->row_chunk >= tri->rows && tri->col_chunk >= tri->cols &&
                               (reinterpret_cast<uintptr_t>(tri->base) & 127u) == 0;
-    if (tensor_core_path(desc) && plain_layout && (desc->c_hidden == 128 || desc->c_hidden == 256)) {
-        // the wide (2c) form exists only in the folded kernel, which takes no residual but z itself
-        const bool wide = desc->c_hidden != desc->c;
-        const bool folded_ok = (desc->flags & TRIMUL_FLAG_INPLACE_NORM_STAGE3) == 0 && (residual == nullptr || residual == z);
-        if (!wide || folded_ok) return run_fast_tm2(desc, z, tri, w, out, residual, st, status);
+    // the folded kernel takes no residual but z itself
+    const bool folded_ok = plain_layout && (desc->flags & TRIMUL_FLAG_INPLACE_NORM_STAGE3) == 0 &&
+                           (residual == nullptr || residual == z);
+    if (tensor_core_path(desc) && plain_layout) {
+        if (desc->c_hidden == 128)
+            return folded_ok ? run_fold_tm2<128, 128>(desc, z, tri, w, out, residual, st, status)
+                             : run_inplace_tm2(desc, z, tri, w, out, residual, st, status);
+        if (desc->c_hidden == 256 && folded_ok) return run_fold_tm2<128, 256>(desc, z, tri, w, out, residual, st, status);
+    }
+    // h = 64 (in the step, c = 64, B = 2, N = 512: 53 us, 74 with both LayerNorms in place; c = 128, N = 448: 42 us, 345 on the
+    // warp-MMA kernel).  The folded kernel reads the LayerNorm vectors 16 bytes at a time, those below one float at a time.
+    if (folded_ok && desc->c_hidden == 64 && aligned16(w->ln_in_weight) && aligned16(w->ln_in_bias) &&
+        aligned16(w->ln_out_weight) && aligned16(w->ln_out_bias)) {
+        if (tensor_core_path(desc)) return run_fold_tm2<128, 64>(desc, z, tri, w, out, residual, st, status);
+        if (narrow_tensor_core_path(desc)) return run_fold_tm2<64, 64>(desc, z, tri, w, out, residual, st, status);
     }
     if (wide_tensor_core_path(desc) && plain_layout) return run_wide_tm2(desc, z, tri, w, out, residual, st, status);
     if (narrow_tensor_core_path(desc) && plain_layout) return run_narrow_tm2(desc, z, tri, w, out, residual, st, status);

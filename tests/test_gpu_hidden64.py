@@ -1,4 +1,4 @@
-"""64 hidden channels: the stacked-operand tensor-core kernels (c = 64 and 128) against the CUDA-core kernels of
+"""64 hidden channels: the tensor-core kernels of stages 1 and 3 (c = 64 and 128), stage 1 against the CUDA-core kernel of
 the same stage, at the edges of the 128-position tiles, over masks, chunked planes and unaligned LayerNorm
 vectors."""
 
@@ -52,3 +52,55 @@ def test_stage1_matches_the_cuda_core_kernel(dev, c, B, N, mask_kind, layout, ou
         assert O.rel_rms(got.cpu(), ref.cpu()) <= 4e-3
         assert ((got - ref).abs() <= 2 ** -7 * ref.abs() + 1e-3 * ref.abs().max()).all()
     assert read_status(dev)[0] == 0
+
+
+@pytest.mark.parametrize("c", [64, 128])
+@pytest.mark.parametrize("B,N,residual,scale", [
+    (1, 1, "z", False), (2, 33, None, False), (1, 128, "z", True), (1, 129, None, True), (3, 127, "z", False),
+    (1, 255, "other", False), (1, 300, "z", True)])
+def test_stage3_against_64_bits(dev, c, B, N, residual, scale):
+    """The folded last stage, and what takes over where it does not apply (another residual, LayerNorm vectors that
+    are not 16-byte aligned), against the stage in 64 bits on the same bf16 operands."""
+    from miniworld_engine_b200 import _lib, read_status, stages as S
+    import ctypes as C
+    w = O.make_weights(c, 41, affine="random", h=64).to(torch.bfloat16)
+    kw = weights_dict(w, torch.bfloat16, dev)
+    g = torch.Generator().manual_seed(42)
+    z = torch.randn(B, N, N, c, generator=g).bfloat16()
+    tri = (torch.randn(B * 64, N, N, generator=g) + 0.5).bfloat16()
+    ds = ((torch.rand(B, 1, N, c, generator=g) > 0.25).float() / 0.75).bfloat16() if scale else None
+    res = {None: None, "z": z, "other": torch.randn(B, N, N, c, generator=g).bfloat16()}[residual]
+
+    d64 = lambda t: t.double()
+    ln = lambda x, gm, bt, eps: torch.nn.functional.layer_norm(x, x.shape[-1:], d64(gm), d64(bt), eps)
+    zn = ln(d64(z), w.ln_pair_weight, w.ln_pair_bias, w.eps_in)
+    tn = ln(d64(tri).view(B, 64, N, N).permute(0, 2, 3, 1), w.ln_out_weight, w.ln_out_bias, w.eps_out)
+    upd = torch.sigmoid(zn @ d64(w.to_gate).T) * (tn @ d64(w.to_out).T)
+    if ds is not None:
+        upd = upd * d64(ds)
+
+    t = S.alloc_planes(B * 64, N, N, torch.bfloat16, dev, fill=float("nan"))
+    S.dense_to_planes(t, tri.to(dev))
+    zd, lib = z.to(dev), _lib.load()
+    rd = zd if residual == "z" else None if res is None else res.to(dev)
+    dsd = None if ds is None else ds.to(dev)
+    errs = []
+    for move in (False, True):
+        k = dict(kw)
+        if move:
+            for n in ("ln_in_w", "ln_in_b", "ln_out_w", "ln_out_b"):
+                k[n] = shifted(k[n])
+        ws, _ = S._weights_struct(c, z.dtype, device=dev, c_hidden=64, c_proj=64, **k)
+        desc = _lib.make_desc(B, N, c, c_hidden=64, dtype=_lib.DTYPE_BF16, direction=_lib.OUTGOING, eps_in=w.eps_in,
+                              eps_out=w.eps_out, drop_scale=None if dsd is None else dsd.data_ptr())
+        out = torch.empty_like(zd)
+        _lib.check(lib.trimul_b200_tm2(C.byref(desc), zd.data_ptr(), C.byref(t.struct()), C.byref(ws), out.data_ptr(),
+                                       None if rd is None else rd.data_ptr(),
+                                       torch.cuda.current_stream(dev).cuda_stream, None), "tm2")
+        y = out.cpu().double()
+        ref = upd if res is None else upd + d64(res)
+        errs.append(float((y - ref).norm() / ref.norm()))
+    assert read_status(dev)[0] == 0
+    # roundings to bf16 (1.1e-3 rms each): the folded weights or the normalised operands, twice; the output, with a
+    # scale and a residual once more each; the hardware tanh adds 2.5e-4 of the gate
+    assert max(errs) <= 5e-3, errs
