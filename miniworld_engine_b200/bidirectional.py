@@ -35,9 +35,9 @@ import torch
 import torch.nn as nn
 
 from . import _lib
-from .functional import (_dtype_code, _mask_bytes, _pinned_weights, _require_cuda, _require_no_grad,
-                         _status_words, _workspace)
-from .module import PinnedLayerNormParams, _lecun_trunc_normal_
+from .functional import (_dtype_code, _mask_bytes, _on_device, _pinned_weights, _plain, _require_cuda, _require_no_grad,
+                         _status_words, _stream_handle, _workspace)
+from .module import PinnedLayerNormParams, _lecun_trunc_normal_, _param, _sub
 
 __all__ = ["bidir_trimul_forward", "bidirectional_triangle_multiplicative_update_b200",
            "BidirectionalTriangleMultiplicationB200"]
@@ -72,10 +72,11 @@ def bidir_trimul_forward(
         raise ValueError(f"w_out must be [{d}, {h2}] and w_gate [{d}, {d}]")
     if mask is not None and tuple(mask.shape) != (B, N):
         raise ValueError(f"mask must be [B, N], got {tuple(mask.shape)}")
-    _require_no_grad("bidir_trimul_forward", x, ln_in_weight, ln_in_bias, w_left, w_left_gate, w_right, w_right_gate,
-                     ln_out_weight, ln_out_bias, w_gate, w_out)
+    if torch.is_grad_enabled():
+        _require_no_grad("bidir_trimul_forward", x, ln_in_weight, ln_in_bias, w_left, w_left_gate, w_right, w_right_gate,
+                         ln_out_weight, ln_out_bias, w_gate, w_out)
     _require_cuda(x, "x")
-    x = x.detach().contiguous()
+    x = _plain(x)
     mask_kind, mask_u8 = _lib.MASK_NONE, None
     if mask is not None:
         _require_cuda(mask, "mask")
@@ -88,14 +89,14 @@ def bidir_trimul_forward(
     nbytes = C.c_size_t()
     _lib.check(lib.trimul_b200_bidir_workspace_bytes(C.byref(desc), C.byref(nbytes)),
                "trimul_b200_bidir_workspace_bytes")
-    with torch.cuda.device(x.device):
-        ws = _workspace(x.device, nbytes.value)
+    with _on_device(x.device):
+        stream = _stream_handle(x.device)
+        ws = _workspace(x.device, nbytes.value, stream)
         out = torch.empty_like(x)
-        st = _status_words(x.device)
         rc = lib.trimul_b200_forward_bidir(
             C.byref(desc), x.data_ptr(), mask_u8.data_ptr() if mask_u8 is not None else None, C.byref(w),
-            out.data_ptr(), 1 if add_residual else 0, ws.data_ptr(), ws.numel(),
-            torch.cuda.current_stream(x.device).cuda_stream, st.data_ptr())
+            out.data_ptr(), 1 if add_residual else 0, ws.data_ptr(), ws.numel(), stream,
+            _status_words(x.device).data_ptr())
     _lib.check(rc, "trimul_b200_forward_bidir")
     for t in keep:      # parameter copies made above must outlive the enqueued kernels
         t.record_stream(torch.cuda.current_stream(x.device))
@@ -160,17 +161,20 @@ class BidirectionalTriangleMultiplicationB200(nn.Module):
             for lin in (self.to_left_gate, self.to_right_gate, self.to_gate, self.to_out):
                 lin.weight.zero_()
 
-    @torch.no_grad()
     def block(self, pair: torch.Tensor, mask: torch.Tensor | None = None, *, add_residual: bool = True,
               plain_kernels: bool = False) -> torch.Tensor:
+        if torch.is_grad_enabled():
+            with torch.no_grad():
+                return self.block(pair, mask, add_residual=add_residual, plain_kernels=plain_kernels)
+        ln_in, ln_out = _sub(self, "ln_pair"), _sub(self, "ln_out")
         return bidir_trimul_forward(
             pair, mask,
-            ln_in_weight=self.ln_pair.weight, ln_in_bias=self.ln_pair.bias,
-            w_left=self.to_left.weight, w_left_gate=self.to_left_gate.weight,
-            w_right=self.to_right.weight, w_right_gate=self.to_right_gate.weight,
-            ln_out_weight=self.ln_out.weight, ln_out_bias=self.ln_out.bias,
-            w_gate=self.to_gate.weight, w_out=self.to_out.weight,
-            eps_in=self.ln_pair.eps, eps_out=self.ln_out.eps,
+            ln_in_weight=_param(ln_in, "weight"), ln_in_bias=_param(ln_in, "bias"),
+            w_left=_param(_sub(self, "to_left"), "weight"), w_left_gate=_param(_sub(self, "to_left_gate"), "weight"),
+            w_right=_param(_sub(self, "to_right"), "weight"), w_right_gate=_param(_sub(self, "to_right_gate"), "weight"),
+            ln_out_weight=_param(ln_out, "weight"), ln_out_bias=_param(ln_out, "bias"),
+            w_gate=_param(_sub(self, "to_gate"), "weight"), w_out=_param(_sub(self, "to_out"), "weight"),
+            eps_in=ln_in.eps, eps_out=ln_out.eps,
             add_residual=add_residual, plain_kernels=plain_kernels)
 
     def forward(self, pair: torch.Tensor, mask: torch.Tensor | None = None,

@@ -22,7 +22,7 @@
 // The bounded waits of this kernel are out of line (mbar_wait<true>): measured 2-7 % faster than
 // the inlined polling loops (N = 768 ... 2048).
 //
-// kScatter = true: the output rows are split into row chunks of d_row_chunk rows and chunk d is
+// Scatter = ScatterMaps: the output rows are split into row chunks of d_row_chunk rows and chunk d is
 // stored through destination map d (the multi-GPU exchange of the channel-sharded contraction,
 // done by the producing kernel's own TMA stores: chunk d is GPU d's slab of rows).
 #pragma once
@@ -37,11 +37,12 @@ constexpr int kC2StageBytes = 2 * kC2HalfBytes;          // this CTA's A half + 
 constexpr int kC2SmemBytes = kC2Stages * kC2StageBytes + kCtStagingBytes + kCtBarBytes;
 constexpr int kC2EpiBarrier = 1;
 
-template <bool kScatter>
+template <typename Scatter>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kCtThreads, 1)
 contract2_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ CUtensorMap tmD, const ContractParams p,
-                       const __grid_constant__ ScatterMaps sc) {
+                       const __grid_constant__ Scatter sc) {
+    constexpr bool kScatter = std::is_same<Scatter, ScatterMaps>::value;
     extern __shared__ __align__(1024) uint8_t smem[];
     // (a misaligned dynamic shared-memory base would be the same in both CTAs: uniform exit)
     if ((smem_u32(smem) & 1023u) != 0u) {
@@ -208,7 +209,7 @@ contract2_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                 fence_proxy_async_smem();
                 named_barrier_sync(kC2EpiBarrier, 128);
                 if (leader_thread) {
-                    if (kScatter)   // this CTA's 128 rows lie inside one destination's row chunk
+                    if constexpr (kScatter)   // this CTA's 128 rows lie inside one destination's row chunk
                         tma_store_4d(&sc.map[row_d / p.d_row_chunk], buf, col0, row_d % p.d_row_chunk, plane, 0);
                     else
                         tma_store_4d(&tmD, buf, col0 % p.d_col_chunk, row_d % p.d_row_chunk, plane,

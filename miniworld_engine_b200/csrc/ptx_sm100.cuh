@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace trimul {
 
 // ---------------------------------------------------------------------------------------
@@ -220,6 +222,7 @@ constexpr int kMaxDest = 8;
 struct ScatterMaps {
     CUtensorMap map[kMaxDest];
 };
+struct NoScatter {};      // takes its place in the kernels that do not scatter: a kilobyte less to copy per launch
 
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");

@@ -30,7 +30,7 @@
 //   acc_empty[b]  in the leader, 16 arrivals: the set's eight epilogue warps of each CTA (remote arrive)
 //   w_all         in the leader, 2 arrivals: each CTA's weights are loaded and halved
 //
-// kScatter = true: a warp's 32 planes are stored in segments of planes_per_dest planes (16 or 32),
+// Scatter = ScatterMaps: a warp's 32 planes are stored in segments of planes_per_dest planes (16 or 32),
 // each through the tensor map of the destination buffer that holds those planes — the multi-GPU
 // exchange of the channel-sharded contraction, done by this kernel's own TMA stores.
 #pragma once
@@ -57,13 +57,14 @@ constexpr int kP1LnBarrier = 2;        // 2, 3: the two LayerNorm groups
 constexpr int kP1EpiBarrier = 4;       // 4, 5: the eight epilogue warps of accumulator set 0, 1
 static_assert(kP1SmemBytes <= 232448, "stage 1 shared memory exceeds the 227 KB a CTA may use");
 
-template <bool kScatter>
+template <typename Scatter>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kP1Threads, 1)
 tm1_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmWl,
                       const __grid_constant__ CUtensorMap tmWlg, const __grid_constant__ CUtensorMap tmWr,
                       const __grid_constant__ CUtensorMap tmWrg, const __grid_constant__ CUtensorMap tmA,
                       const __grid_constant__ CUtensorMap tmB, const __grid_constant__ Tm1Params p,
-                      const __grid_constant__ ScatterMaps scA, const __grid_constant__ ScatterMaps scB) {
+                      const __grid_constant__ Scatter scA, const __grid_constant__ Scatter scB) {
+    constexpr bool kScatter = std::is_same<Scatter, ScatterMaps>::value;
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0u) {
         // both CTAs of a pair see the same offset, so both leave here and nobody waits for the other
@@ -324,7 +325,7 @@ tm1_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             if (lane == 0) {
                 const int col0 = t0 + half * 64;
                 if (col0 < p.n_run) {
-                    if (kScatter) {
+                    if constexpr (kScatter) {
                         // the warp's 32 planes in segments of one destination's share
                         const ScatterMaps* sm = is_leader ? &scA : &scB;
                         const int seg = p.planes_per_dest < 32 ? p.planes_per_dest : 32;

@@ -320,11 +320,14 @@ int run_fast_tm1(const trimul_desc* d, const void* z, const uint8_t* mask, const
                  const trimul_planes* a, const trimul_planes* b, cudaStream_t st, int32_t* status, int n_dest = 0) {
     const bool inc = d->direction == TRIMUL_INCOMING;
     CUtensorMap tmZ, tmW[4];
+    const bool pair = (d->flags & TRIMUL_FLAG_SINGLE_CTA_STAGE1) == 0 && sm_count() >= 2;
     {
+        // a lone CTA loads whole 128-position tiles, a CTA of a pair its 64 positions
         const uint64_t dims[4] = {128, (uint64_t)d->N, (uint64_t)d->rows, (uint64_t)d->B};
         const uint64_t strides[3] = {128, (uint64_t)d->N * 128, (uint64_t)d->rows * d->N * 128};
-        const uint32_t box_out[4] = {64, 128, 1, 1};
-        const uint32_t box_in[4] = {64, 1, 128, 1};
+        const uint32_t pos = pair ? 64 : 128;
+        const uint32_t box_out[4] = {64, pos, 1, 1};
+        const uint32_t box_in[4] = {64, 1, pos, 1};
         if (!encode_bf16(&tmZ, z, 4, dims, strides, inc ? box_in : box_out, 128)) return TRIMUL_E_CUDA;
     }
     const void* ws[4] = {w->w_left, w->w_left_gate, w->w_right, w->w_right_gate};
@@ -356,21 +359,16 @@ int run_fast_tm1(const trimul_desc* d, const void* z, const uint8_t* mask, const
     p.status = status;
     const int grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
     const bool overlap = overlap_launches(d->flags);
-    if ((d->flags & TRIMUL_FLAG_SINGLE_CTA_STAGE1) == 0 && sm_count() >= 2) {
+    if (pair) {
         // CTA pairs: each CTA holds one side's weights and normalises 64 positions of a tile
-        CUtensorMap tmZh, tmA, tmB;
-        ScatterMaps scA{}, scB{};
-        const uint64_t dims[4] = {128, (uint64_t)d->N, (uint64_t)d->rows, (uint64_t)d->B};
-        const uint64_t strides[3] = {128, (uint64_t)d->N * 128, (uint64_t)d->rows * d->N * 128};
-        const uint32_t box_out[4] = {64, 64, 1, 1};
-        const uint32_t box_in[4] = {64, 1, 64, 1};
-        if (!encode_bf16(&tmZh, z, 4, dims, strides, inc ? box_in : box_out, 128)) return TRIMUL_E_CUDA;
+        CUtensorMap tmA, tmB;
         const int pairs = p.total_tiles < sm_count() / 2 ? p.total_tiles : sm_count() / 2;
         for (int k = 0; k < 2; ++k) {
             p.step_q[k] = (k + 1) * pairs / p.tiles_per_fixed;
             p.step_r[k] = (k + 1) * pairs % p.tiles_per_fixed;
         }
         if (n_dest > 0) {
+            ScatterMaps scA{}, scB{};
             // one epilogue warp stores 64 positions x 32 planes, in segments of one destination's share
             const uint32_t seg = planes_per_dest < 32 ? planes_per_dest : 32;
             for (int k = 0; k < n_dest; ++k) {
@@ -379,16 +377,16 @@ int run_fast_tm1(const trimul_desc* d, const void* z, const uint8_t* mask, const
             }
             tmA = scA.map[0];
             tmB = scB.map[0];
-            if (!ensure_smem(tm1_pair_sm100_kernel<true>, kP1SmemBytes)) return TRIMUL_E_CUDA;
-            return launch_stage(tm1_pair_sm100_kernel<true>, 2 * pairs, kP1Threads, kP1SmemBytes, st, overlap, tmZh,
+            if (!ensure_smem(tm1_pair_sm100_kernel<ScatterMaps>, kP1SmemBytes)) return TRIMUL_E_CUDA;
+            return launch_stage(tm1_pair_sm100_kernel<ScatterMaps>, 2 * pairs, kP1Threads, kP1SmemBytes, st, overlap, tmZ,
                                 tmW[0], tmW[1], tmW[2], tmW[3], tmA, tmB, p, scA, scB);
         }
         // one epilogue warp stores 64 positions x 32 planes
         if (!encode_planes(&tmA, *a, planes, 64, 1, 32)) return TRIMUL_E_CUDA;
         if (!encode_planes(&tmB, *b, planes, 64, 1, 32)) return TRIMUL_E_CUDA;
-        if (!ensure_smem(tm1_pair_sm100_kernel<false>, kP1SmemBytes)) return TRIMUL_E_CUDA;
-        return launch_stage(tm1_pair_sm100_kernel<false>, 2 * pairs, kP1Threads, kP1SmemBytes, st, overlap, tmZh,
-                            tmW[0], tmW[1], tmW[2], tmW[3], tmA, tmB, p, scA, scB);
+        if (!ensure_smem(tm1_pair_sm100_kernel<NoScatter>, kP1SmemBytes)) return TRIMUL_E_CUDA;
+        return launch_stage(tm1_pair_sm100_kernel<NoScatter>, 2 * pairs, kP1Threads, kP1SmemBytes, st, overlap, tmZ,
+                            tmW[0], tmW[1], tmW[2], tmW[3], tmA, tmB, p, NoScatter{}, NoScatter{});
     }
     // lone CTAs: all four weight matrices per SM, results staged in shared memory and TMA-stored
     if (n_dest > 0) return TRIMUL_E_UNSUPPORTED;       // only the pair kernel scatters
@@ -540,7 +538,7 @@ bool fast_contract_ok(const trimul_planes* a, const trimul_planes* b, const trim
 int run_fast_contract(int planes, const trimul_planes* a, const trimul_planes* b, const trimul_planes* t,
                       cudaStream_t st, int32_t* status, bool pair, uint32_t flags, int n_dest = 0) {
     CUtensorMap tmA, tmB, tmD;
-    ScatterMaps sc{};
+    ScatterMaps sc;
     if (!encode_planes(&tmA, *a, planes, kCtBK, kCtBM, 1)) return TRIMUL_E_CUDA;
     if (!encode_planes(&tmB, *b, planes, kCtBK, pair ? 128 : kCtBN, 1)) return TRIMUL_E_CUDA;
     for (int k = 0; k < n_dest; ++k)
@@ -566,13 +564,13 @@ int run_fast_contract(int planes, const trimul_planes* a, const trimul_planes* b
         const int clusters = pair_tiles < max_clusters ? (int)pair_tiles : max_clusters;
         const bool overlap = overlap_launches(flags);
         if (n_dest > 0) {
-            if (!ensure_smem(contract2_sm100_kernel<true>, kC2SmemBytes)) return TRIMUL_E_CUDA;
-            return launch_stage(contract2_sm100_kernel<true>, 2 * clusters, kCtThreads, kC2SmemBytes, st, overlap, tmA,
+            if (!ensure_smem(contract2_sm100_kernel<ScatterMaps>, kC2SmemBytes)) return TRIMUL_E_CUDA;
+            return launch_stage(contract2_sm100_kernel<ScatterMaps>, 2 * clusters, kCtThreads, kC2SmemBytes, st, overlap, tmA,
                                 tmB, tmD, p, sc);
         }
-        if (!ensure_smem(contract2_sm100_kernel<false>, kC2SmemBytes)) return TRIMUL_E_CUDA;
-        return launch_stage(contract2_sm100_kernel<false>, 2 * clusters, kCtThreads, kC2SmemBytes, st, overlap, tmA,
-                            tmB, tmD, p, sc);
+        if (!ensure_smem(contract2_sm100_kernel<NoScatter>, kC2SmemBytes)) return TRIMUL_E_CUDA;
+        return launch_stage(contract2_sm100_kernel<NoScatter>, 2 * clusters, kCtThreads, kC2SmemBytes, st, overlap, tmA,
+                            tmB, tmD, p, NoScatter{});
     }
     if (n_dest > 0) return TRIMUL_E_UNSUPPORTED;
     const int64_t total = (int64_t)planes * p.tiles_m * p.tiles_n;
