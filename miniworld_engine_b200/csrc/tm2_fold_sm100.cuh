@@ -332,6 +332,20 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             const int s = it & 1;
             const uint32_t ph = (it >> 1) & 1u;
             const int zs = it % kG2ZStages;
+            // this position's drop-scale values (it is column j0 + row of z row r, any r)
+            const __nv_bfloat16* ds_row = nullptr;
+            if (kDropScale) {
+                const int j0 = (tile % p.tiles_per_row) * kT2P;
+                const int b = (tile / p.tiles_per_row) / p.rows;
+                if (j0 + row < p.N) ds_row = fp.drop_scale + ((size_t)b * p.N + j0 + row) * kC + grp * (kC / 2);
+            }
+            // the scales of two chunks are fetched two chunks ahead, the first ones while the UMMAs run: fetched where
+            // they are used, each chunk waits for L2 (B = 2, N = 256: the stage 43.6 us instead of 39.7)
+            auto fetch_ds = [&](int c8) {
+                return kDropScale && ds_row != nullptr && c8 < kC / 16 ? __ldg(reinterpret_cast<const uint4*>(ds_row) + c8)
+                                                                      : make_uint4(0u, 0u, 0u, 0u);
+            };
+            uint4 dsA = fetch_ds(0), dsB = fetch_ds(1);
             bool ok = true;
             if (leader) {
                 ok = mbar_wait<true>(&acc_full[s], ph, abort_flag, p.status, kStageIdTm2, 400 + s) &&
@@ -351,28 +365,17 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             // kC = 128: the group's half is a sub-tile; kC = 64: the second four 16-byte chunks of the only one
             uint8_t* tile_row = sZ + zs * L::kZBytes + (kC == 128 ? grp * kT2SubTile : 0) + row * 128;
             const int chunk0 = kC == 128 ? 0 : grp * 4;
-            // this position's drop-scale values (it is column j0 + row of z row r, any r)
-            const __nv_bfloat16* ds_row = nullptr;
-            if (kDropScale) {
-                const int j0 = (tile % p.tiles_per_row) * kT2P;
-                const int b = (tile / p.tiles_per_row) / p.rows;
-                if (j0 + row < p.N) ds_row = fp.drop_scale + ((size_t)b * p.N + j0 + row) * kC + grp * (kC / 2);
-            }
             // 8 output channels (one 16-byte chunk) at a time; the TMEM loads of the next 8 are in
             // flight while the current 8 get their statistics, are gated, rounded and written over the
             // z tile.  The loop stays rolled to keep the code small.
-            auto emit8 = [&](int c8, const uint32_t (&rg)[8], const uint32_t (&rp)[8]) {
+            auto emit8 = [&](int c8, const uint32_t (&rg)[8], const uint32_t (&rp)[8], const uint4& dv) {
                 uint4* dst = reinterpret_cast<uint4*>(tile_row + (((chunk0 + c8) ^ (row & 7)) << 4));
                 uint32_t res[4] = {0u, 0u, 0u, 0u};
                 if (kResidualIsZ) {
                     const uint4 rv = *dst;
                     res[0] = rv.x; res[1] = rv.y; res[2] = rv.z; res[3] = rv.w;
                 }
-                uint32_t dsw[4] = {0u, 0u, 0u, 0u};
-                if (kDropScale && ds_row != nullptr) {
-                    const uint4 dv = __ldg(reinterpret_cast<const uint4*>(ds_row + c8 * 8));
-                    dsw[0] = dv.x; dsw[1] = dv.y; dsw[2] = dv.z; dsw[3] = dv.w;
-                }
+                const uint32_t dsw[4] = {dv.x, dv.y, dv.z, dv.w};
                 uint32_t o[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -399,7 +402,10 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                 tmem_ld_wait();
                 tmem_ld_32x8(t_g + (c8 + 1) * 8, rgB);
                 tmem_ld_32x8(t_g + 128 + (c8 + 1) * 8, rpB);
-                emit8(c8, rgA, rpA);
+                const uint4 dvA = dsA, dvB = dsB;
+                dsA = fetch_ds(c8 + 2);
+                dsB = fetch_ds(c8 + 3);
+                emit8(c8, rgA, rpA, dvA);
                 tmem_ld_wait();
                 if (c8 + 2 < kC / 16) {
                     tmem_ld_32x8(t_g + (c8 + 2) * 8, rgA);
@@ -410,7 +416,7 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&acc_empty[s]);
                 }
-                emit8(c8 + 1, rgB, rpB);
+                emit8(c8 + 1, rgB, rpB, dvB);
             }
             fence_proxy_async_smem();      // result half -> visible to the TMA store (async proxy)
             __syncwarp();
