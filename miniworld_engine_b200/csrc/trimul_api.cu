@@ -741,39 +741,32 @@ int run_narrow_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri
                         tmWg, tmWo, tmOut, tmTri, tmRes, np);
 }
 
-// c = h = 256: weights streamed through shared memory (tm2_wide_sm100.cuh)
+// c = h = 256: CTA pairs, each CTA holding half of both folded matrices (tm2_wide_sm100.cuh)
 int run_wide_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri, const trimul_weights* w, void* out,
                  const void* residual, cudaStream_t st, int32_t* status) {
+    if ((int64_t)d->B * d->rows * ((d->N + kT2P - 1) / kT2P) > 0x3fffffff) return TRIMUL_E_UNSUPPORTED;
     CUtensorMap tmZ, tmWg, tmWo, tmOut, tmTri;
     const uint64_t dims[4] = {kW2C, (uint64_t)d->N, (uint64_t)d->rows, (uint64_t)d->B};
     const uint64_t strides[3] = {kW2C, (uint64_t)d->N * kW2C, (uint64_t)d->rows * d->N * kW2C};
     const uint32_t box[4] = {64, 128, 1, 1};
+    const uint32_t obox[4] = {32, 32, 1, 1};
     if (!encode_bf16(&tmZ, z, 4, dims, strides, box, 128)) return TRIMUL_E_CUDA;
-    if (!encode_bf16(&tmOut, out, 4, dims, strides, box, 128)) return TRIMUL_E_CUDA;
+    if (!encode_bf16(&tmOut, out, 4, dims, strides, obox, 64)) return TRIMUL_E_CUDA;
     const uint64_t wdims[2] = {kW2C, kW2C};
     const uint64_t wstrides[1] = {kW2C};
     const uint32_t wbox[2] = {64, 128};
     if (!encode_bf16(&tmWg, w->w_gate, 2, wdims, wstrides, wbox, 128)) return TRIMUL_E_CUDA;
     if (!encode_bf16(&tmWo, w->w_out, 2, wdims, wstrides, wbox, 128)) return TRIMUL_E_CUDA;
-    if (!encode_planes(&tmTri, *tri, d->B * kW2C, 64, 1, 128)) return TRIMUL_E_CUDA;
+    if (!encode_planes(&tmTri, *tri, d->B * kW2C, 64, 1, 64)) return TRIMUL_E_CUDA;
     Tm2WideParams wp = {};
-    Tm2Params& p = wp.base;
-    p.B = d->B; p.rows = d->rows; p.N = d->N;
-    p.tiles_per_row = (d->N + kT2P - 1) / kT2P;
-    const int64_t total = (int64_t)d->B * d->rows * p.tiles_per_row;
-    if (total > 0x7fffffff) return TRIMUL_E_UNSUPPORTED;
-    p.total_tiles = (int)total;
-    p.gamma_in = w->ln_in_weight; p.beta_in = w->ln_in_bias;
-    p.gamma_out = w->ln_out_weight; p.beta_out = w->ln_out_bias;
-    p.eps_in = d->eps_in; p.eps_out = d->eps_out;
-    p.has_residual = residual != nullptr;
-    p.status = status;
+    wp.base = tm2_params(d, w, residual, status);
     wp.residual = static_cast<const __nv_bfloat16*>(residual);
     wp.drop_scale = static_cast<const __nv_bfloat16*>(desc_drop_scale(d));
-    const int grid = p.total_tiles < sm_count() ? p.total_tiles : sm_count();
+    const int pairs = (wp.base.total_tiles + 1) / 2;
+    const int clusters = pairs < sm_count() / 2 ? pairs : sm_count() / 2;
     if (!ensure_smem(tm2_wide_sm100_kernel, kW2SmemBytes)) return TRIMUL_E_CUDA;
-    return launch_stage(tm2_wide_sm100_kernel, grid, kW2Threads, kW2SmemBytes, st, overlap_launches(d->flags), tmZ, tmWg,
-                        tmWo, tmOut, tmTri, wp);
+    return launch_stage(tm2_wide_sm100_kernel, 2 * clusters, kW2Threads, kW2SmemBytes, st, overlap_launches(d->flags), tmZ,
+                        tmWg, tmWo, tmOut, tmTri, wp);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -977,7 +970,7 @@ int trimul_b200_tm2(const trimul_desc* desc, const void* z, const trimul_planes*
         if (tensor_core_path(desc)) return run_fold_tm2<128, 64>(desc, z, tri, w, out, residual, st, status);
         if (narrow_tensor_core_path(desc)) return run_fold_tm2<64, 64>(desc, z, tri, w, out, residual, st, status);
     }
-    if (wide_tensor_core_path(desc) && plain_layout) return run_wide_tm2(desc, z, tri, w, out, residual, st, status);
+    if (wide_tensor_core_path(desc) && plain_layout && sm_count() >= 2) return run_wide_tm2(desc, z, tri, w, out, residual, st, status);
     if (narrow_tensor_core_path(desc) && plain_layout) return run_narrow_tm2(desc, z, tri, w, out, residual, st, status);
     const void* mats[2] = {w->w_gate, w->w_out};
     if (wmma_ok(desc, mats, 2)) return run_wmma_tm2(desc, z, tri, w, out, residual, st);

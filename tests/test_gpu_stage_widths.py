@@ -1,6 +1,6 @@
-"""64 hidden channels: the tensor-core kernels of stages 1 and 3 (c = 64 and 128), stage 1 against the CUDA-core kernel of
-the same stage, at the edges of the 128-position tiles, over masks, chunked planes and unaligned LayerNorm
-vectors."""
+"""Stages 1 and 3 on the tensor cores at widths other than c = h = 128: stage 1 against the CUDA-core kernel of the
+same stage, stage 3 against 64 bits, at the edges of the 128-position tiles (odd tile counts among them), over masks,
+residuals, dropout scales, chunked planes and unaligned LayerNorm vectors."""
 
 import pytest
 import torch
@@ -54,32 +54,32 @@ def test_stage1_matches_the_cuda_core_kernel(dev, c, B, N, mask_kind, layout, ou
     assert read_status(dev)[0] == 0
 
 
-@pytest.mark.parametrize("c", [64, 128])
+@pytest.mark.parametrize("c,h", [(64, 64), (128, 64), (256, 256)])
 @pytest.mark.parametrize("B,N,residual,scale", [
     (1, 1, "z", False), (2, 33, None, False), (1, 128, "z", True), (1, 129, None, True), (3, 127, "z", False),
-    (1, 255, "other", False), (1, 300, "z", True)])
-def test_stage3_against_64_bits(dev, c, B, N, residual, scale):
+    (1, 255, "other", False), (1, 300, "z", True), (1, 385, None, False)])
+def test_stage3_against_64_bits(dev, c, h, B, N, residual, scale):
     """The folded last stage, and what takes over where it does not apply (another residual, LayerNorm vectors that
     are not 16-byte aligned), against the stage in 64 bits on the same bf16 operands."""
     from miniworld_engine_b200 import _lib, read_status, stages as S
     import ctypes as C
-    w = O.make_weights(c, 41, affine="random", h=64).to(torch.bfloat16)
+    w = O.make_weights(c, 41, affine="random", h=h).to(torch.bfloat16)
     kw = weights_dict(w, torch.bfloat16, dev)
     g = torch.Generator().manual_seed(42)
     z = torch.randn(B, N, N, c, generator=g).bfloat16()
-    tri = (torch.randn(B * 64, N, N, generator=g) + 0.5).bfloat16()
+    tri = (torch.randn(B * h, N, N, generator=g) + 0.5).bfloat16()
     ds = ((torch.rand(B, 1, N, c, generator=g) > 0.25).float() / 0.75).bfloat16() if scale else None
     res = {None: None, "z": z, "other": torch.randn(B, N, N, c, generator=g).bfloat16()}[residual]
 
     d64 = lambda t: t.double()
     ln = lambda x, gm, bt, eps: torch.nn.functional.layer_norm(x, x.shape[-1:], d64(gm), d64(bt), eps)
     zn = ln(d64(z), w.ln_pair_weight, w.ln_pair_bias, w.eps_in)
-    tn = ln(d64(tri).view(B, 64, N, N).permute(0, 2, 3, 1), w.ln_out_weight, w.ln_out_bias, w.eps_out)
+    tn = ln(d64(tri).view(B, h, N, N).permute(0, 2, 3, 1), w.ln_out_weight, w.ln_out_bias, w.eps_out)
     upd = torch.sigmoid(zn @ d64(w.to_gate).T) * (tn @ d64(w.to_out).T)
     if ds is not None:
         upd = upd * d64(ds)
 
-    t = S.alloc_planes(B * 64, N, N, torch.bfloat16, dev, fill=float("nan"))
+    t = S.alloc_planes(B * h, N, N, torch.bfloat16, dev, fill=float("nan"))
     S.dense_to_planes(t, tri.to(dev))
     zd, lib = z.to(dev), _lib.load()
     rd = zd if residual == "z" else None if res is None else res.to(dev)
@@ -90,8 +90,8 @@ def test_stage3_against_64_bits(dev, c, B, N, residual, scale):
         if move:
             for n in ("ln_in_w", "ln_in_b", "ln_out_w", "ln_out_b"):
                 k[n] = shifted(k[n])
-        ws, _ = S._weights_struct(c, z.dtype, device=dev, c_hidden=64, c_proj=64, **k)
-        desc = _lib.make_desc(B, N, c, c_hidden=64, dtype=_lib.DTYPE_BF16, direction=_lib.OUTGOING, eps_in=w.eps_in,
+        ws, _ = S._weights_struct(c, z.dtype, device=dev, c_hidden=h, c_proj=h, **k)
+        desc = _lib.make_desc(B, N, c, c_hidden=h, dtype=_lib.DTYPE_BF16, direction=_lib.OUTGOING, eps_in=w.eps_in,
                               eps_out=w.eps_out, drop_scale=None if dsd is None else dsd.data_ptr())
         out = torch.empty_like(zd)
         _lib.check(lib.trimul_b200_tm2(C.byref(desc), zd.data_ptr(), C.byref(t.struct()), C.byref(ws), out.data_ptr(),
