@@ -39,7 +39,10 @@
 //
 // kDropScale: the row-broadcast dropout scale of the reference module in training mode multiplies
 // the block output before the residual (a template parameter: the inference instantiations carry
-// no trace of it).
+// no trace of it).  The scale depends on the column only, so a CTA walks down a column block and keeps the block's
+// scale tile in shared memory (in place of the third z buffer for c = 128): read from global memory, one position
+// per thread, it touched 32 lines per load.  Measured, whole block: c = 128, B = 2, N = 256 74.7 -> 71.7 us,
+// N = 768 322 -> 304, N = 1500 1559 -> 1405; c = 64, B = 2, N = 256 60 -> 45.
 //
 // kH = 256 is the last stage of the BIDIRECTIONAL block (bidirectional.py:150-156): tri has 256
 // channel planes per batch ([outgoing | incoming]), LayerNorm_out runs over all 256 and Wo is
@@ -59,9 +62,11 @@ namespace trimul {
 constexpr int kG2Threads = 640;
 constexpr int kG2EpiThreads = 256;      // warps 4..11, two groups of 128
 constexpr int kG2StatThreads = 128;     // each of the two statistics groups
-// kC = channels of z and out (64, 128), kH = channels of tri (64, 128, 256)
-template <int kC, int kH>
+// kC = channels of z and out (64, 128), kH = channels of tri (64, 128, 256); kDropScale: with a dropout scale
+template <int kC, int kH, bool kDropScale>
 struct G2Layout {
+    // The scale tile [128 positions][kC] of a column block is kept in shared memory, except beside the weights of kH = 256
+    static constexpr bool kScaleTile = kDropScale && kH != 256;
     static constexpr int kSlotCh = kH < 128 ? kH : 128;          // channel planes per tri slot
     static constexpr int kSlots = kH / kSlotCh;                  // tri slots per tile
     static constexpr int kWSub = kC * 128;                       // [kC output channels][64 k] of a weight matrix
@@ -69,17 +74,18 @@ struct G2Layout {
     static constexpr int kZBytes = kC / 64 * kT2SubTile;         // z tile: 64-channel sub-tiles
     static constexpr int kTSub = kSlotCh * 128;                  // [channels][64 positions] of a tri slot
     static constexpr int kTBytes = 2 * kTSub;
-    static constexpr int kZStages = kC == 64 ? 6 : kH == 256 ? 2 : 3;
+    static constexpr int kZStages = kC == 64 ? 6 : kH == 256 || kScaleTile ? 2 : 3;
     static constexpr int kTStages = kTBytes == 32768 ? 2 : 4;
     static constexpr int kOffZ = kWBytes;
     static constexpr int kOffT = kOffZ + kZStages * kZBytes;     // tri ring; once a tile's tri data is dead the
                                                                  // first 2 KB of its last slot hold [128 positions]
                                                                  // (r_in, t_in, r_out, t_out)
-    static constexpr int kOffConst = kOffT + kTStages * kTBytes; // [2 matrices][64 channel pairs] (s0, s1, b0, b1)
+    static constexpr int kOffScale = kOffT + kTStages * kTBytes;
+    static constexpr int kOffConst = kOffScale + (kScaleTile ? kZBytes : 0);   // [2 matrices][64 channel pairs] (s0, s1, b0, b1)
     static constexpr int kOffBars = kOffConst + 2048;
-    static constexpr int kSmemBytes = kOffBars + 384;
+    static constexpr int kSmemBytes = kOffBars + 512;
     static_assert(kSmemBytes <= 232448, "folded stage 3 shared memory exceeds the 227 KB a CTA may use");
-    static_assert((10 + 4 * kZStages + 3 * kTStages) * 8 + 8 <= 384, "barrier block too small");
+    static_assert((12 + 4 * kZStages + 3 * kTStages) * 8 + 8 <= 512, "barrier block too small");
 };
 constexpr int kG2StatInBarrier = 2;
 constexpr int kG2StatOutBarrier = 3;
@@ -96,14 +102,15 @@ template <bool kResidualIsZ, int kC, int kH, bool kDropScale>
 __global__ void __launch_bounds__(kG2Threads, 1)
 tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmWg,
                       const __grid_constant__ CUtensorMap tmWo, const __grid_constant__ CUtensorMap tmOut,
-                      const __grid_constant__ CUtensorMap tmTri, const Tm2FoldParams fp) {
+                      const __grid_constant__ CUtensorMap tmTri, const __grid_constant__ CUtensorMap tmScale,
+                      const Tm2FoldParams fp) {
     const Tm2Params& p = fp.base;
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0u) {
         if (threadIdx.x == 0) report_timeout(p.status, kStageIdTm2, 900);
         return;
     }
-    using L = G2Layout<kC, kH>;
+    using L = G2Layout<kC, kH, kDropScale>;
     constexpr int kG2ZStages = L::kZStages, kTS = L::kTStages, kSlots = L::kSlots, kSlotCh = L::kSlotCh;
     constexpr int kCSub = kC / 64;              // 64-channel sub-tiles of z and out
     uint8_t* sW = smem;
@@ -123,7 +130,9 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     uint64_t* acc_empty = acc_full + 2;         // [2] (8 arrivals)
     uint64_t* stat_in = acc_empty + 2;          // [2] z statistics written into the tri buffer (128 arrivals)
     uint64_t* stat_out = stat_in + 2;           // [2] tri statistics written (128 arrivals)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stat_out + 2);
+    uint64_t* ds_full = stat_out + 2;           // scale tile landed
+    uint64_t* ds_empty = ds_full + 1;           // the last tile of its column block is through the epilogue (8 arrivals)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ds_empty + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
@@ -149,6 +158,8 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             mbar_init(&stat_in[s], kG2StatThreads);
             mbar_init(&stat_out[s], kG2StatThreads);
         }
+        mbar_init(ds_full, 1);
+        mbar_init(ds_empty, 8);
         *abort_flag = 0;
         fence_mbarrier_init();
         tma_prefetch_desc(&tmZ);
@@ -167,20 +178,40 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     griddep_wait();
     griddep_launch_dependents();
 
+    // This CTA's tiles.  Usually every gridDim.x-th in row order; with a scale tile a contiguous run in COLUMN order
+    // (column block, then rows), because the scale is the same for all rows of a column block: it is loaded once or twice
+    // per CTA instead of being read from L2 by every thread of every tile.
+    const int t_begin = L::kScaleTile ? (int)((long long)p.total_tiles * blockIdx.x / gridDim.x) : (int)blockIdx.x;
+    const int t_end = L::kScaleTile ? (int)((long long)p.total_tiles * (blockIdx.x + 1) / gridDim.x) : p.total_tiles;
+    const int t_step = L::kScaleTile ? 1 : (int)gridDim.x;
+    auto place = [&](int tile, int& b, int& r, int& j0) {
+        if (L::kScaleTile) {
+            const int q = tile / p.rows;
+            r = tile - q * p.rows;
+            b = q / p.tiles_per_row;
+            j0 = (q - b * p.tiles_per_row) * kT2P;
+        } else {
+            const int br = tile / p.tiles_per_row;
+            j0 = (tile - br * p.tiles_per_row) * kT2P;
+            b = br / p.rows;
+            r = br - b * p.rows;
+        }
+    };
+
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
             mbar_arrive_expect_tx(w_full, L::kWBytes);
             for (int kh = 0; kh < kCSub; ++kh) tma_load_2d(sW + kh * L::kWSub, &tmWg, w_full, kh * 64, 0);
             for (int kh = 0; kh < kH / 64; ++kh) tma_load_2d(sW + (kCSub + kh) * L::kWSub, &tmWo, w_full, kh * 64, 0);
+            int column = -1;
+            uint32_t columns = 0;
             uint32_t it = 0;
-            for (int tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
+            for (int tile = t_begin; tile < t_end; tile += t_step, ++it) {
                 const int zs = it % kG2ZStages;
                 const uint32_t zph = (it / kG2ZStages) & 1u;
-                const int j0 = (tile % p.tiles_per_row) * kT2P;
-                const int br = tile / p.tiles_per_row;
-                const int r = br % p.rows;
-                const int b = br / p.rows;
+                int b, r, j0;
+                place(tile, b, r, j0);
                 bool okp = true;
                 for (int h = 0; h < kSlots; ++h) {
                     // tri slot of this part of the channels: slots are used round-robin, use n = u / kTS
@@ -207,6 +238,14 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                 mbar_arrive_expect_tx(&z_full[zs], L::kZBytes);
                 uint8_t* dz = sZ + zs * L::kZBytes;
                 for (int ks = 0; ks < kCSub; ++ks) tma_load_4d(dz + ks * kT2SubTile, &tmZ, &z_full[zs], ks * 64, j0, r, b);
+                if (L::kScaleTile && tile / p.rows != column) {      // first tile of a column block
+                    column = tile / p.rows;
+                    if (!mbar_wait<true>(ds_empty, (columns & 1u) ^ 1u, abort_flag, p.status, kStageIdTm2, 120)) break;
+                    ++columns;
+                    mbar_arrive_expect_tx(ds_full, L::kZBytes);
+                    for (int ks = 0; ks < kCSub; ++ks)
+                        tma_load_4d(smem + L::kOffScale + ks * kT2SubTile, &tmScale, ds_full, ks * 64, j0, 0, b);
+                }
             }
         }
         __syncwarp();
@@ -218,7 +257,7 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             bool ok = mbar_wait<true>(w_ready, 0, abort_flag, p.status, kStageIdTm2, 200);
             tcgen05_fence_after();
             uint32_t it = 0;
-            for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x, ++it) {
+            for (int tile = t_begin; ok && tile < t_end; tile += t_step, ++it) {
                 const int s = it & 1;
                 const uint32_t ph = (it >> 1) & 1u;
                 // accumulator pair `s` was last used by tile it-2
@@ -269,13 +308,11 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         // ------------------------------------------------------------------ store warp
         if (lane == 0) {
             uint32_t it = 0;
-            for (int tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
+            for (int tile = t_begin; tile < t_end; tile += t_step, ++it) {
                 const int s = it % kG2ZStages;
                 const uint32_t ph = (it / kG2ZStages) & 1u;
-                const int j0 = (tile % p.tiles_per_row) * kT2P;
-                const int br = tile / p.tiles_per_row;
-                const int r = br % p.rows;
-                const int b = br / p.rows;
+                int b, r, j0;
+                place(tile, b, r, j0);
                 const uint8_t* src = sZ + s * L::kZBytes;
                 if (!mbar_wait<true>(&box_ready[2 * s], ph, abort_flag, p.status, kStageIdTm2, 600 + s)) break;
                 if (kC == 128) {
@@ -327,31 +364,36 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         const uint32_t lane_bits = (uint32_t)(q * 32) << 16;
         const ulonglong2* cG = reinterpret_cast<const ulonglong2*>(sConst) + grp * (kC / 4);
         const ulonglong2* cO = cG + 64;
-        uint32_t it = 0;
-        for (int tile = blockIdx.x; run && tile < p.total_tiles; tile += gridDim.x, ++it) {
+        uint32_t it = 0, columns = 0;
+        int column = -1;
+        for (int tile = t_begin; run && tile < t_end; tile += t_step, ++it) {
             const int s = it & 1;
             const uint32_t ph = (it >> 1) & 1u;
             const int zs = it % kG2ZStages;
-            // this position's drop-scale values (it is column j0 + row of z row r, any r)
+            // this position's drop-scale values (it is column j0 + row of z row r, any r): from the scale tile, or, where
+            // there is no room for it, from global memory, two chunks fetched two chunks ahead
             const __nv_bfloat16* ds_row = nullptr;
-            if (kDropScale) {
-                const int j0 = (tile % p.tiles_per_row) * kT2P;
-                const int b = (tile / p.tiles_per_row) / p.rows;
+            if (kDropScale && !L::kScaleTile) {
+                int b, r, j0;
+                place(tile, b, r, j0);
                 if (j0 + row < p.N) ds_row = fp.drop_scale + ((size_t)b * p.N + j0 + row) * kC + grp * (kC / 2);
             }
-            // the scales of two chunks are fetched two chunks ahead, the first ones while the UMMAs run: fetched where
-            // they are used, each chunk waits for L2 (B = 2, N = 256: the stage 43.6 us instead of 39.7)
+            const uint8_t* scale_row = smem + L::kOffScale + (kC == 128 ? grp * kT2SubTile : 0) + row * 128;
             auto fetch_ds = [&](int c8) {
                 return kDropScale && ds_row != nullptr && c8 < kC / 16 ? __ldg(reinterpret_cast<const uint4*>(ds_row) + c8)
                                                                       : make_uint4(0u, 0u, 0u, 0u);
             };
             uint4 dsA = fetch_ds(0), dsB = fetch_ds(1);
+            const bool new_column = L::kScaleTile && tile / p.rows != column;
+            if (new_column) column = tile / p.rows;
             bool ok = true;
             if (leader) {
                 ok = mbar_wait<true>(&acc_full[s], ph, abort_flag, p.status, kStageIdTm2, 400 + s) &&
                      mbar_wait<true>(&stat_in[s], ph, abort_flag, p.status, kStageIdTm2, 410 + s) &&
                      mbar_wait<true>(&stat_out[s], ph, abort_flag, p.status, kStageIdTm2, 420 + s);
+                if (new_column) ok = ok && mbar_wait<true>(ds_full, columns & 1u, abort_flag, p.status, kStageIdTm2, 430);
             }
+            if (new_column) ++columns;
             if (!named_barrier_all(bar_id, 128, ok)) break;
             tcgen05_fence_after();
             if (e == 0) TRIMUL_STAMP(4, it, 0);
@@ -375,7 +417,9 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                     const uint4 rv = *dst;
                     res[0] = rv.x; res[1] = rv.y; res[2] = rv.z; res[3] = rv.w;
                 }
-                const uint32_t dsw[4] = {dv.x, dv.y, dv.z, dv.w};
+                uint4 dt = dv;
+                if (L::kScaleTile) dt = *reinterpret_cast<const uint4*>(scale_row + (((chunk0 + c8) ^ (row & 7)) << 4));
+                const uint32_t dsw[4] = {dt.x, dt.y, dt.z, dt.w};
                 uint32_t o[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -387,7 +431,7 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                     float g0, g1;
                     f2_unpack(hg, g0, g1);
                     o[k] = f2_to_bf16x2(f2_fma(ho, f2_pack(tanh_fast(g0), tanh_fast(g1)), ho));
-                    if (kDropScale && ds_row != nullptr)   // the scale multiplies the rounded block output, like `out * scale`
+                    if (L::kScaleTile || (kDropScale && ds_row != nullptr))   // the scale multiplies the rounded block output, like `out * scale`
                         o[k] = f2_to_bf16x2(f2_mul(f2_from_bf16x2(o[k]), f2_from_bf16x2(dsw[k])));
                     if (kResidualIsZ)   // the reference rounds the block output to bf16 before `out + pair`
                         o[k] = f2_to_bf16x2(f2_add(f2_from_bf16x2(o[k]), f2_from_bf16x2(res[k])));
@@ -421,13 +465,14 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
             fence_proxy_async_smem();      // result half -> visible to the TMA store (async proxy)
             __syncwarp();
             if (lane == 0) mbar_arrive(&box_ready[2 * zs + grp]);
+            if (L::kScaleTile && (tile + 1 == t_end || (tile + 1) / p.rows != column) && lane == 0) mbar_arrive(ds_empty);
             if (e == 0) TRIMUL_STAMP(4, it, 1);
         }
     } else if (warp < 16) {
         // ------------------------------------------------------------------ statistics of the z tile
         const int pos = threadIdx.x - 384;             // 0..127, row of the tile
         uint32_t it = 0;
-        for (int tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x, ++it) {
+        for (int tile = t_begin; tile < t_end; tile += t_step, ++it) {
             const int s = it & 1;
             const int zs = it % kG2ZStages;
             if (!group_wait<true>(&z_full[zs], (it / kG2ZStages) & 1u, pos == 0, kG2StatInBarrier, kG2StatThreads, abort_flag,
@@ -461,7 +506,7 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         const float inv_c = 1.0f / (float)kH;
         uint32_t it = 0;
         bool alive = true;
-        for (int tile = blockIdx.x; alive && tile < p.total_tiles; tile += gridDim.x, ++it) {
+        for (int tile = t_begin; alive && tile < t_end; tile += t_step, ++it) {
             const int s = it & 1;
             uint32_t sh[4] = {0u, 0u, 0u, 0u};
             f32x2 nsh[4] = {0ull, 0ull, 0ull, 0ull}, a[4] = {0ull, 0ull, 0ull, 0ull}, qq[4] = {0ull, 0ull, 0ull, 0ull};

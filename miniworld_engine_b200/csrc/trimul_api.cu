@@ -649,7 +649,6 @@ Tm2Params tm2_params(const trimul_desc* d, const trimul_weights* w, const void* 
 template <int kC, int kH>
 int run_fold_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri, const trimul_weights* w, void* out,
                  const void* residual, cudaStream_t st, int32_t* status) {
-    using L = G2Layout<kC, kH>;
     if ((int64_t)d->B * d->rows * ((d->N + kT2P - 1) / kT2P) > 0x7fffffff) return TRIMUL_E_UNSUPPORTED;
     CUtensorMap tmZ, tmWg, tmWo, tmOut, tmTri;
     const uint64_t dims[4] = {kC, (uint64_t)d->N, (uint64_t)d->rows, (uint64_t)d->B};
@@ -662,22 +661,29 @@ int run_fold_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri, 
     const uint32_t wbox[2] = {64, kC};
     if (!encode_bf16(&tmWg, w->w_gate, 2, wdims, wstrides, wbox, 128)) return TRIMUL_E_CUDA;
     if (!encode_bf16(&tmWo, w->w_out, 2, wodims, wostrides, wbox, 128)) return TRIMUL_E_CUDA;
-    if (!encode_planes(&tmTri, *tri, d->B * kH, 64, 1, L::kSlotCh)) return TRIMUL_E_CUDA;
+    if (!encode_planes(&tmTri, *tri, d->B * kH, 64, 1, G2Layout<kC, kH, false>::kSlotCh)) return TRIMUL_E_CUDA;
     Tm2FoldParams fp;
     fp.base = tm2_params(d, w, residual, status);
     fp.residual_is_z = residual != nullptr;
     fp.drop_scale = static_cast<const __nv_bfloat16*>(desc_drop_scale(d));
     const int grid = fp.base.total_tiles < sm_count() ? fp.base.total_tiles : sm_count();
-    auto launch = [&](auto kernel) {
-        if (!ensure_smem(kernel, L::kSmemBytes)) return (int)TRIMUL_E_CUDA;
-        return launch_stage(kernel, grid, kG2Threads, L::kSmemBytes, st, overlap_launches(d->flags), tmZ, tmWg, tmWo, tmOut,
-                            tmTri, fp);
+    CUtensorMap tmScale = tmZ;
+    if (fp.drop_scale != nullptr) {
+        const uint64_t sdims[4] = {kC, (uint64_t)d->N, 1, (uint64_t)d->B};
+        const uint64_t sstrides[3] = {kC, (uint64_t)d->N * kC, (uint64_t)d->N * kC};
+        if (!encode_bf16(&tmScale, fp.drop_scale, 4, sdims, sstrides, box, 128)) return TRIMUL_E_CUDA;
+    }
+    auto launch = [&](auto kernel, int smem) {
+        if (!ensure_smem(kernel, smem)) return (int)TRIMUL_E_CUDA;
+        return launch_stage(kernel, grid, kG2Threads, smem, st, overlap_launches(d->flags), tmZ, tmWg, tmWo, tmOut, tmTri,
+                            tmScale, fp);
     };
+    constexpr int kSmem = G2Layout<kC, kH, false>::kSmemBytes, kSmemScale = G2Layout<kC, kH, true>::kSmemBytes;
     if (fp.drop_scale != nullptr)
-        return residual != nullptr ? launch(tm2_fold_sm100_kernel<true, kC, kH, true>)
-                                   : launch(tm2_fold_sm100_kernel<false, kC, kH, true>);
-    return residual != nullptr ? launch(tm2_fold_sm100_kernel<true, kC, kH, false>)
-                               : launch(tm2_fold_sm100_kernel<false, kC, kH, false>);
+        return residual != nullptr ? launch(tm2_fold_sm100_kernel<true, kC, kH, true>, kSmemScale)
+                                   : launch(tm2_fold_sm100_kernel<false, kC, kH, true>, kSmemScale);
+    return residual != nullptr ? launch(tm2_fold_sm100_kernel<true, kC, kH, false>, kSmem)
+                               : launch(tm2_fold_sm100_kernel<false, kC, kH, false>, kSmem);
 }
 
 // c = h = 128 with a residual that is not z (or on request): both LayerNorms in place (tm2_sm100.cuh)
@@ -964,9 +970,8 @@ int trimul_b200_tm2(const trimul_desc* desc, const void* z, const trimul_planes*
         if (desc->c_hidden == 256 && folded_ok) return run_fold_tm2<128, 256>(desc, z, tri, w, out, residual, st, status);
     }
     // h = 64 (in the step, c = 64, B = 2, N = 512: 53 us, 74 with both LayerNorms in place; c = 128, N = 448: 42 us, 345 on the
-    // warp-MMA kernel).  The folded kernel reads the LayerNorm vectors 16 bytes at a time, those below one float at a time.
-    if (folded_ok && desc->c_hidden == 64 && aligned16(w->ln_in_weight) && aligned16(w->ln_in_bias) &&
-        aligned16(w->ln_out_weight) && aligned16(w->ln_out_bias)) {
+    // warp-MMA kernel)
+    if (folded_ok && desc->c_hidden == 64) {
         if (tensor_core_path(desc)) return run_fold_tm2<128, 64>(desc, z, tri, w, out, residual, st, status);
         if (narrow_tensor_core_path(desc)) return run_fold_tm2<64, 64>(desc, z, tri, w, out, residual, st, status);
     }

@@ -54,10 +54,10 @@ def test_stage1_matches_the_cuda_core_kernel(dev, c, B, N, mask_kind, layout, ou
     assert read_status(dev)[0] == 0
 
 
-@pytest.mark.parametrize("c,h", [(64, 64), (128, 64), (256, 256)])
+@pytest.mark.parametrize("c,h", [(64, 64), (128, 64), (128, 128), (128, 256), (256, 256)])
 @pytest.mark.parametrize("B,N,residual,scale", [
     (1, 1, "z", False), (2, 33, None, False), (1, 128, "z", True), (1, 129, None, True), (3, 127, "z", False),
-    (1, 255, "other", False), (1, 300, "z", True), (1, 385, None, False)])
+    (1, 255, "other", False), (1, 300, "z", True), (3, 130, "z", True), (1, 385, None, False)])
 def test_stage3_against_64_bits(dev, c, h, B, N, residual, scale):
     """The folded last stage, and what takes over where it does not apply (another residual, LayerNorm vectors that
     are not 16-byte aligned), against the stage in 64 bits on the same bf16 operands."""
