@@ -937,11 +937,12 @@ __device__ __forceinline__ void row_stats(const uint8_t* tile, int sub_bytes, in
 // Fold one row (output channel n) of a weight matrix that lies in shared memory as `nsub` swizzled
 // 64-column sub-tiles (`sub_bytes` apart): w[k] <- bf16(w[k] * gamma[k] / 2).  Returns the sum of the rounded row and
 // 0.5 * sum_k w[k] * beta[k].  gamma and beta may lie at any float address.
-__device__ __forceinline__ float4 ldg_f4_any(const float* p) {
-    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) return __ldg(reinterpret_cast<const float4*>(p));
+template <bool kAligned> __device__ __forceinline__ float4 ldg_f4(const float* p) {
+    if (kAligned) return __ldg(reinterpret_cast<const float4*>(p));
     return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
 }
-__device__ __forceinline__ void fold_row_smem(uint8_t* wbase, int sub_bytes, int n, const float* gamma,
+template <bool kAligned>
+__device__ __forceinline__ void fold_row_any(uint8_t* wbase, int sub_bytes, int n, const float* gamma,
                                               const float* beta, int nsub, float& s, float& bias) {
     float ssum = 0.f, bsum = 0.f;
     const uint32_t swz = (uint32_t)(n & 7);
@@ -952,10 +953,10 @@ __device__ __forceinline__ void fold_row_smem(uint8_t* wbase, int sub_bytes, int
             uint4* ptr = reinterpret_cast<uint4*>(wbase + kh * sub_bytes + n * 128 + ((((uint32_t)j) ^ swz) << 4));
             const uint4 v = *ptr;
             const int k0 = kh * 64 + j * 8;
-            const float4 g0 = ldg_f4_any(gamma + k0);
-            const float4 g1 = ldg_f4_any(gamma + k0 + 4);
-            const float4 b0 = ldg_f4_any(beta + k0);
-            const float4 b1 = ldg_f4_any(beta + k0 + 4);
+            const float4 g0 = ldg_f4<kAligned>(gamma + k0);
+            const float4 g1 = ldg_f4<kAligned>(gamma + k0 + 4);
+            const float4 b0 = ldg_f4<kAligned>(beta + k0);
+            const float4 b1 = ldg_f4<kAligned>(beta + k0 + 4);
             const float ga[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
             const float be[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
             const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
@@ -974,6 +975,16 @@ __device__ __forceinline__ void fold_row_smem(uint8_t* wbase, int sub_bytes, int
     s = ssum;
     bias = 0.5f * bsum;
 }
-
+__device__ __noinline__ void fold_row_unaligned(uint8_t* wbase, int sub_bytes, int n, const float* gamma, const float* beta,
+                                                int nsub, float& s, float& bias) {
+    fold_row_any<false>(wbase, sub_bytes, n, gamma, beta, nsub, s, bias);
+}
+__device__ __forceinline__ void fold_row_smem(uint8_t* wbase, int sub_bytes, int n, const float* gamma,
+                                              const float* beta, int nsub, float& s, float& bias) {
+    if (((reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) & 15u) == 0)
+        fold_row_any<true>(wbase, sub_bytes, n, gamma, beta, nsub, s, bias);
+    else
+        fold_row_unaligned(wbase, sub_bytes, n, gamma, beta, nsub, s, bias);
+}
 
 }  // namespace trimul
