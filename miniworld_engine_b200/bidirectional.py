@@ -165,7 +165,11 @@ class BidirectionalTriangleMultiplicationB200(nn.Module):
               plain_kernels: bool = False) -> torch.Tensor:
         if torch.is_grad_enabled():
             with torch.no_grad():
-                return self.block(pair, mask, add_residual=add_residual, plain_kernels=plain_kernels)
+                return self._block_no_grad(pair, mask, add_residual, plain_kernels)
+        return self._block_no_grad(pair, mask, add_residual, plain_kernels)
+
+    def _block_no_grad(self, pair, mask, add_residual, plain_kernels) -> torch.Tensor:
+        """The body of ``block``, apart from it so that an override of ``block`` is not entered a second time."""
         ln_in, ln_out = _sub(self, "ln_pair"), _sub(self, "ln_out")
         return bidir_trimul_forward(
             pair, mask,

@@ -122,7 +122,11 @@ class TriangleMultiplicationB200(nn.Module):
         ``drop_scale`` ``[B, 1, L, D]`` multiplies it before the residual is added)."""
         if torch.is_grad_enabled():
             with torch.no_grad():
-                return self.block(pair, mask, residual=residual, plain_kernels=plain_kernels, drop_scale=drop_scale)
+                return self._block_no_grad(pair, mask, residual, plain_kernels, drop_scale)
+        return self._block_no_grad(pair, mask, residual, plain_kernels, drop_scale)
+
+    def _block_no_grad(self, pair, mask, residual, plain_kernels, drop_scale) -> torch.Tensor:
+        """The body of ``block``, apart from it so that an override of ``block`` is not entered a second time."""
         ln_in, ln_out = _sub(self, "ln_pair"), _sub(self, "ln_out")
         return F_b200.trimul_forward(
             pair, mask, outgoing=self.outgoing,
