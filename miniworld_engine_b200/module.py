@@ -65,8 +65,12 @@ def _param(module: nn.Module, name: str) -> torch.Tensor:
 
 
 def _sub(module: nn.Module, name: str) -> nn.Module:
+    """``getattr(module, name)``; a registered submodule that neither the class nor the instance shadows is read from the
+    module's own table."""
     sub = module._modules.get(name)
-    return getattr(module, name) if sub is None else sub
+    if sub is None or name in module.__dict__ or hasattr(type(module), name):
+        return getattr(module, name)
+    return sub
 
 
 _PLAIN_TYPES = (nn.Linear, PinnedLayerNormParams)

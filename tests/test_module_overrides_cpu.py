@@ -3,6 +3,7 @@
 
 import pytest
 import torch
+import torch.nn.utils.parametrize
 
 from miniworld_engine_b200 import BidirectionalTriangleMultiplicationB200, TriangleMultiplicationB200, bidirectional, functional
 
@@ -57,3 +58,24 @@ def test_a_wrapper_around_the_bound_block_runs_once(calls, base, grad):
         y = m(x)                      # forward calls the wrapper
     assert len(entered) == 1 and len(calls) == 1
     assert torch.equal(y, 2 * x)
+
+
+@pytest.mark.parametrize("base", MODULES.values(), ids=MODULES)
+def test_submodules_and_parameters_are_what_the_attributes_say(calls, base):
+    """A property of a subclass, an attribute of the instance and a parametrised weight take precedence over the
+    registered submodule or parameter of that name."""
+    other = torch.nn.Linear(8, 8, bias=False)
+
+    class Shared(base):
+        @property
+        def to_gate(self):
+            return other
+
+    m = Shared(8)
+    m.__dict__["to_out"] = torch.nn.Linear(m.to_left.weight.shape[0], 8, bias=False)
+    torch.nn.utils.parametrize.register_parametrization(m.to_left, "weight", torch.nn.Tanh())
+    m.block(torch.ones(1, 3, 3, 8))
+    assert calls[0]["w_gate"] is other.weight
+    assert calls[0]["w_out"] is m.__dict__["to_out"].weight
+    assert torch.equal(calls[0]["w_left"], m.to_left.weight) and calls[0]["w_left"] is not m.to_left.parametrizations.weight.original
+    assert calls[0]["w_right"] is m.to_right.weight
