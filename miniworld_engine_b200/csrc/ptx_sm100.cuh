@@ -869,26 +869,10 @@ __device__ __forceinline__ void ln_load_affine_quad(f32x2 (&gb)[16], const float
 }
 
 // gamma and beta of a lane's channels for ln_rows_warp, from global memory: lane chunk j = lane & 7 owns
-// channels [64 s + 8 j, 64 s + 8 j + 8) of every sub-tile s.
+// channels [64 s + 8 j, 64 s + 8 j + 8) of every sub-tile s.  4-byte loads, once per thread and launch: the vectors may lie at
+// any float address (a view into a flat parameter buffer).
 template <int kSub>
 __device__ __forceinline__ void ln_load_affine(f32x2 (&gb)[8 * kSub], const float* gamma, const float* beta, int lane) {
-    const int j = lane & 7;
-#pragma unroll
-    for (int s = 0; s < kSub; ++s) {
-        const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + 64 * s + 8 * j));
-        const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma + 64 * s + 8 * j + 4));
-        const float4 b0 = __ldg(reinterpret_cast<const float4*>(beta + 64 * s + 8 * j));
-        const float4 b1 = __ldg(reinterpret_cast<const float4*>(beta + 64 * s + 8 * j + 4));
-        gb[4 * s + 0] = f2_pack(g0.x, g0.y); gb[4 * s + 1] = f2_pack(g0.z, g0.w);
-        gb[4 * s + 2] = f2_pack(g1.x, g1.y); gb[4 * s + 3] = f2_pack(g1.z, g1.w);
-        gb[4 * kSub + 4 * s + 0] = f2_pack(b0.x, b0.y); gb[4 * kSub + 4 * s + 1] = f2_pack(b0.z, b0.w);
-        gb[4 * kSub + 4 * s + 2] = f2_pack(b1.x, b1.y); gb[4 * kSub + 4 * s + 3] = f2_pack(b1.z, b1.w);
-    }
-}
-
-// The same with 4-byte loads, for kernels whose callers may pass LayerNorm vectors at any float address.
-template <int kSub>
-__device__ __forceinline__ void ln_load_affine_scalar(f32x2 (&gb)[8 * kSub], const float* gamma, const float* beta, int lane) {
 #pragma unroll
     for (int s = 0; s < kSub; ++s)
 #pragma unroll

@@ -197,7 +197,7 @@ tm1_narrow_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_co
         const int rr = lane / (32 / kRows);
         f32x2 gb[16];
         if constexpr (kSub == 1) ln_load_affine_quad(gb, p.gamma, p.beta, lane);
-        else ln_load_affine_scalar<kSub>(gb, p.gamma, p.beta, lane);
+        else ln_load_affine<kSub>(gb, p.gamma, p.beta, lane);
         const int first = blockIdx.x + lg * stride;
         uint32_t it = lg;
         Tm1Cursor cur;

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from oracle import trimul_oracle as O
-from tests._util import weights_dict
+from tests._util import forward_kwargs, weights_dict
 
 pytestmark = pytest.mark.gpu
 
@@ -104,3 +104,35 @@ def test_stage3_against_64_bits(dev, c, h, B, N, residual, scale):
     # roundings to bf16 (1.1e-3 rms each): the folded weights or the normalised operands, twice; the output, with a
     # scale and a residual once more each; the hardware tanh adds 2.5e-4 of the gate
     assert max(errs) <= 5e-3, errs
+
+
+@pytest.mark.parametrize("single_cta", [False, True], ids=["pair", "lone"])
+@pytest.mark.parametrize("c", [64, 128, 256])
+def test_stage1_takes_layernorm_vectors_at_any_float_address(dev, c, single_cta):
+    """c = h: the same values at an address that is not 16-byte aligned give the same bits."""
+    from miniworld_engine_b200 import read_status, stages as S
+    B, N = 2, 130
+    kw = weights_dict(O.make_weights(c, 51, affine="random"), torch.bfloat16, dev)
+    z = O.make_input(B, N, c, 52).bfloat16().to(dev)
+    outs = []
+    for move in (False, True):
+        k = {n: shifted(v) if move and n.startswith("ln_") else v for n, v in kw.items()}
+        assert k["ln_in_w"].data_ptr() % 16 == (4 if move else 0)
+        a, b = (S.alloc_planes(B * c, N, N, torch.bfloat16, dev, fill=float("nan")) for _ in range(2))
+        S.tm1(z, None, k, a, b, outgoing=False, single_cta=single_cta)
+        outs.append([S.planes_to_dense(s) for s in (a, b)])
+    assert read_status(dev)[0] == 0
+    for ref, got in zip(*outs):
+        assert not torch.isnan(ref.float()).any() and torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("c", [64, 128, 256])
+def test_a_block_takes_layernorm_vectors_at_any_float_address(dev, c):
+    from miniworld_engine_b200 import read_status, trimul_forward
+    kw = forward_kwargs(O.make_weights(c, 53, affine="random"), torch.bfloat16, dev)
+    z = O.make_input(1, 70, c, 54).bfloat16().to(dev)
+    ref, got = (trimul_forward(z, None, outgoing=True, residual=z,
+                               **{n: shifted(v) if move and n.startswith("ln_") else v for n, v in kw.items()})
+                for move in (False, True))
+    assert read_status(dev)[0] == 0
+    assert torch.equal(got, ref)
