@@ -587,7 +587,31 @@ __device__ __forceinline__ uint32_t gate2_bf16(float hp0, float hg0, float hp1, 
     return f2_to_bf16x2(f2_fma(hp, f2_pack(tanh_fast(hg0), tanh_fast(hg1)), hp));
 }
 
-// the same from UNHALVED p and g (kernels that stream their weights and cannot halve them once)
+// p * sigmoid(g) for two values from halves, rounded to a bf16x2 word.  kFp32: the gate to 1e-6 of its own size (1e-5 at
+// g = -80), as p/2 times 2 / (1 + 2^(-2 log2(e) g/2)).  tanh.approx is off by up to 2.5e-4 of the gate's FULL scale, which
+// leaves nothing of a nearly shut gate (sigmoid(-8) = 3.4e-4); the fp32 form takes two MUFU operations instead of one and is
+// for the widths whose gates were evaluated in fp32 before they had a tcgen05 kernel.  (Flush to zero: a power below 2^-126
+// does not show beside 1; gates below 2^-126, at g < -87, become 0.)
+template <bool kFp32>
+__device__ __forceinline__ uint32_t gate_halves_bf16(f32x2 hp, f32x2 hg) {
+    float g0, g1;
+    if constexpr (kFp32) {
+        const f32x2 half2 = f2_pack(0.5f, 0.5f);
+        f2_unpack(f2_mul(hg, f2_pack(-2.885390082f, -2.885390082f)), g0, g1);
+        float e0, e1, s0, s1;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(g0));
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(g1));
+        f2_unpack(f2_fma(f2_pack(e0, e1), half2, half2), e0, e1);
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s0) : "f"(e0));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s1) : "f"(e1));
+        return f2_to_bf16x2(f2_mul(hp, f2_pack(s0, s1)));
+    } else {
+        f2_unpack(hg, g0, g1);
+        return f2_to_bf16x2(f2_fma(hp, f2_pack(tanh_fast(g0), tanh_fast(g1)), hp));
+    }
+}
+
+// the same as gate2_bf16 from UNHALVED p and g (kernels that stream their weights and cannot halve them once)
 __device__ __forceinline__ uint32_t gate2_full_bf16(float p0, float g0, float p1, float g1) {
     const f32x2 half2 = f2_pack(0.5f, 0.5f);
     const f32x2 hp = f2_mul(f2_pack(p0, p1), half2);

@@ -10,7 +10,8 @@
 // W_right_gate] for the gates, so lanes 0..63 of the accumulators are the channels of a and lanes
 // 64..127 those of b.  A tile is then 8 kSub UMMAs (K = 64 kSub) into 2 x 128 TMEM columns; the
 // accumulators are double-buffered and the weight matrices stay in shared memory (halved once, exact in
-// bf16, for the tanh form of the gate).
+// bf16, for the half-argument forms of the gate: the hardware tanh for c = 64; for c = 128, where the warp-MMA kernel
+// had expf, the fp32 form, which keeps the bits of nearly shut gates.  It costs 1.8 us of a call at N = 512).
 //
 // What bounds it: HBM (c = 64: z once, a and b once).  LayerNorm and epilogue have the form of the CTA-pair
 // kernel (tm1_pair_sm100.cuh): eight lanes per LayerNorm row with every value read once, and sixteen
@@ -258,8 +259,8 @@ tm1_narrow_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_co
                 uint32_t o[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    o[e] = gate2_bf16(__uint_as_float(rp[2 * e]), __uint_as_float(rg[2 * e]),
-                                      __uint_as_float(rp[2 * e + 1]), __uint_as_float(rg[2 * e + 1]));
+                    o[e] = gate_halves_bf16<kSub == 2>(f2_pack(__uint_as_float(rp[2 * e]), __uint_as_float(rp[2 * e + 1])),
+                                                       f2_pack(__uint_as_float(rg[2 * e]), __uint_as_float(rg[2 * e + 1])));
                 const int chunk = c8 ^ (lane & 7);
                 *reinterpret_cast<uint4*>(box + lane * 128 + (chunk << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
             };

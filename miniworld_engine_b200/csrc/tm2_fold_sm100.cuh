@@ -50,7 +50,9 @@
 // ring (so a tile occupies the whole ring and the z ring is two deep: Wo takes 32 KB more); the
 // projection accumulates over both halves and the tri statistics are summed over both.
 // kH = 64 (c = 64, or a hidden width of half the pair width) has tri slots of 64 channels, four of them; with kC = 64
-// the z ring is six 16 KB tiles deep and the two epilogue groups share the tile's only 64-channel sub-tile.  Measured in
+// the z ring is six 16 KB tiles deep and the two epilogue groups share the tile's only 64-channel sub-tile.  c = 128 with
+// kH = 64 evaluates the gate to fp32 accuracy (gate_halves_bf16), as the warp-MMA kernel before it did (3 us of a
+// call at N = 512).  Measured in
 // the step: c = 64, B = 2, N = 512 53 us instead of 74 with the LayerNorms in place, N = 1024 94 instead of 138;
 // c = 128, h = 64, N = 448 42 instead of 345 on the warp-MMA kernel.
 #pragma once
@@ -428,9 +430,7 @@ tm2_fold_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                                             f2_fma(tin, kg.x, kg.y));
                     const f32x2 ho = f2_fma(f2_pack(__uint_as_float(rp[2 * k]), __uint_as_float(rp[2 * k + 1])), rout,
                                             f2_fma(tout, ko.x, ko.y));
-                    float g0, g1;
-                    f2_unpack(hg, g0, g1);
-                    o[k] = f2_to_bf16x2(f2_fma(ho, f2_pack(tanh_fast(g0), tanh_fast(g1)), ho));
+                    o[k] = gate_halves_bf16<kC == 128 && kH == 64>(ho, hg);
                     if (L::kScaleTile || (kDropScale && ds_row != nullptr))   // the scale multiplies the rounded block output, like `out * scale`
                         o[k] = f2_to_bf16x2(f2_mul(f2_from_bf16x2(o[k]), f2_from_bf16x2(dsw[k])));
                     if (kResidualIsZ)   // the reference rounds the block output to bf16 before `out + pair`

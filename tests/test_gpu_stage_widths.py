@@ -136,3 +136,70 @@ def test_a_block_takes_layernorm_vectors_at_any_float_address(dev, c):
                 for move in (False, True))
     assert read_status(dev)[0] == 0
     assert torch.equal(got, ref)
+
+
+def closed_gates(c, h):
+    """Weights whose gate logits are about -8 (sigmoid(-8) = 3.4e-4): LayerNorm_in has a bias of one, the gate rows a mean of -8/c."""
+    w = O.make_weights(c, 61, affine="random", h=h)
+    w.ln_pair_weight[:], w.ln_pair_bias[:] = 1.0, 1.0
+    g = torch.Generator().manual_seed(62)
+    for m in (w.to_left_gate, w.to_right_gate, w.to_gate):
+        m.copy_(-8.0 / c + 0.05 * torch.randn(m.shape, generator=g) / c ** 0.5)
+    return w.to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("mask_kind", [None, "pair"])
+def test_stage1_keeps_the_bits_of_nearly_shut_gates_at_64_hidden_channels(dev, mask_kind):
+    """c = 128, h = 64.  Against the CUDA-core kernel (the same rounding of x_n, expf): a hardware tanh, off by 2.5e-4 of the
+    gate's full scale, would be off by half the value here."""
+    from miniworld_engine_b200 import read_status, stages as S
+    B, N = 2, 70
+    kw = weights_dict(closed_gates(128, 64), torch.bfloat16, dev)
+    z = O.make_input(B, N, 128, 63).bfloat16().to(dev)
+    mask = None if mask_kind is None else (torch.rand(B, N, N, generator=torch.Generator().manual_seed(64)) > 0.2).to(dev)
+
+    def run(plain):
+        a, b = (S.alloc_planes(B * 64, N, N, torch.bfloat16, dev, fill=float("nan")) for _ in range(2))
+        S.tm1(z, mask, kw, a, b, outgoing=True, plain_kernels=plain)
+        return S.planes_to_dense(a).float().cpu(), S.planes_to_dense(b).float().cpu()
+
+    for got, ref in zip(run(False), run(True)):
+        # one rounding to bf16 each (1.1e-3 rms of the value) and now and then another rounding of an x_n
+        assert 0 < float(ref.abs().max()) < 0.1
+        assert O.rel_rms(got, ref) <= 4e-3
+    assert read_status(dev)[0] == 0
+
+
+@pytest.mark.parametrize("scale", [False, True], ids=["bare", "scaled"])
+def test_stage3_keeps_the_bits_of_nearly_shut_gates_at_64_hidden_channels(dev, scale):
+    """c = 128, h = 64, against the stage in 64 bits on the same bf16 operands."""
+    from miniworld_engine_b200 import _lib, read_status, stages as S
+    from miniworld_engine_b200.functional import _status_words
+    import ctypes as C
+    B, N, c, h = 1, 130, 128, 64
+    w = closed_gates(c, h)
+    kw = weights_dict(w, torch.bfloat16, dev)
+    g = torch.Generator().manual_seed(65)
+    z = torch.randn(B, N, N, c, generator=g).bfloat16()
+    tri = torch.randn(B * h, N, N, generator=g).bfloat16()
+    ds = ((torch.rand(B, 1, N, c, generator=g) > 0.25).float() / 0.75).bfloat16()
+    ln = lambda x, gm, bt, eps: torch.nn.functional.layer_norm(x, x.shape[-1:], gm.double(), bt.double(), eps)
+    zn = ln(z.double(), w.ln_pair_weight, w.ln_pair_bias, w.eps_in)
+    tn = ln(tri.double().view(B, h, N, N).permute(0, 2, 3, 1), w.ln_out_weight, w.ln_out_bias, w.eps_out)
+    ref = torch.sigmoid(zn @ w.to_gate.double().T) * (tn @ w.to_out.double().T)
+    if scale:
+        ref = ref * ds.double()
+    t = S.alloc_planes(B * h, N, N, torch.bfloat16, dev, fill=float("nan"))
+    S.dense_to_planes(t, tri.to(dev))
+    zd, dsd = z.to(dev), ds.to(dev)
+    ws, _ = S._weights_struct(c, z.dtype, device=dev, c_hidden=h, c_proj=h, **kw)
+    desc = _lib.make_desc(B, N, c, c_hidden=h, dtype=_lib.DTYPE_BF16, direction=_lib.OUTGOING, eps_in=w.eps_in,
+                          eps_out=w.eps_out, drop_scale=dsd.data_ptr() if scale else None)
+    out = torch.full_like(zd, float("nan"))
+    _lib.check(_lib.load().trimul_b200_tm2(C.byref(desc), zd.data_ptr(), C.byref(t.struct()), C.byref(ws), out.data_ptr(),
+                                           None, torch.cuda.current_stream(dev).cuda_stream,
+                                           _status_words(dev).data_ptr()), "tm2")
+    # roundings to bf16 of the folded weights (in the logit 8 * 1.1e-3 / sqrt(c), in the projection 1.1e-3), of the output and
+    # of the scaled output
+    assert read_status(dev)[0] == 0
+    assert float((out.cpu().double() - ref).norm() / ref.norm()) <= 5e-3
