@@ -77,7 +77,9 @@ extern "C" {
 #define TRIMUL_FLAG_INPLACE_NORM_STAGE3 16u /* stage 3 with both LayerNorms applied in place in shared
                                          memory before the projections (rounds LN(x) to bf16 like the
                                          reference) instead of the default kernel, which folds them
-                                         into the weights; cross-checking aid, slower               */
+                                         into the weights; cross-checking aid, slower (tcgen05 kernels
+                                         for c == c_hidden == 64 and 128, the warp-MMA or CUDA-core
+                                         kernel at the other widths)                                 */
 #define TRIMUL_FLAG_SERIAL_LAUNCH 32u  /* launch the tensor-core stages without programmatic dependent
                                          launch.  By default a stage may be scheduled while its
                                          predecessor in the stream drains and waits on the device

@@ -975,7 +975,9 @@ int trimul_b200_tm2(const trimul_desc* desc, const void* z, const trimul_planes*
         if (tensor_core_path(desc)) return run_fold_tm2<128, 64>(desc, z, tri, w, out, residual, st, status);
         if (narrow_tensor_core_path(desc)) return run_fold_tm2<64, 64>(desc, z, tri, w, out, residual, st, status);
     }
-    if (wide_tensor_core_path(desc) && plain_layout && sm_count() >= 2) return run_wide_tm2(desc, z, tri, w, out, residual, st, status);
+    // the c = 256 kernel only exists folded: with both LayerNorms in place on request, the warp-MMA kernel below
+    if (wide_tensor_core_path(desc) && plain_layout && sm_count() >= 2 && (desc->flags & TRIMUL_FLAG_INPLACE_NORM_STAGE3) == 0)
+        return run_wide_tm2(desc, z, tri, w, out, residual, st, status);
     if (narrow_tensor_core_path(desc) && plain_layout) return run_narrow_tm2(desc, z, tri, w, out, residual, st, status);
     const void* mats[2] = {w->w_gate, w->w_out};
     if (wmma_ok(desc, mats, 2)) return run_wmma_tm2(desc, z, tri, w, out, residual, st);

@@ -203,3 +203,24 @@ def test_stage3_keeps_the_bits_of_nearly_shut_gates_at_64_hidden_channels(dev, s
     # of the scaled output
     assert read_status(dev)[0] == 0
     assert float((out.cpu().double() - ref).norm() / ref.norm()) <= 5e-3
+
+
+@pytest.mark.parametrize("residual", [None, "z", "other"])
+@pytest.mark.parametrize("c,h", [(256, 256), (128, 64), (128, 256)])
+def test_stage3_with_the_layernorms_in_place_on_request(dev, c, h, residual):
+    """The flag's rounding points (LN(x) to bf16, unchanged weights) are those of the CUDA-core kernel: the outputs are the same
+    but for values that lie on a rounding boundary.  Folded weights (another rounding of every product) change far more."""
+    from miniworld_engine_b200 import read_status, stages as S
+    B, N = 2, 70
+    kw = weights_dict(O.make_weights(c, 71, affine="random", h=h), torch.bfloat16, dev)
+    g = torch.Generator().manual_seed(72)
+    z = torch.randn(B, N, N, c, generator=g).bfloat16().to(dev)
+    t = S.alloc_planes(B * h, N, N, torch.bfloat16, dev, fill=float("nan"))
+    S.dense_to_planes(t, torch.randn(B * h, N, N, generator=g).bfloat16().to(dev))
+    res = {None: None, "z": z, "other": torch.randn(B, N, N, c, generator=g).bfloat16().to(dev)}[residual]
+    plain = S.tm2(z, t, kw, residual=res, plain_kernels=True)
+    asked = S.tm2(z, t, kw, residual=res, inplace_norm=True)
+    assert read_status(dev)[0] == 0
+    # fp32 sums in another order differ by about 1e-6 of the value and a bf16 step is 4e-3 of it: a few in ten thousand of
+    # the roundings of LN(x), and of the outputs, go the other way
+    assert (asked != plain).float().mean() <= 0.02
