@@ -852,7 +852,11 @@ int trimul_b200_tm1(const trimul_desc* desc, const void* z, const uint8_t* mask,
     if (wide_tensor_core_path(desc) && chunks_ok) return run_wide_tm1(desc, z, mask, w, a, b, st, status);
     // h = 64: the stacked-operand kernel (c = 128, bidirectional N = 320: 23 us a call,
     // 159 on the warp-MMA kernel, which keeps the other widths)
-    if ((narrow_tensor_core_path(desc) || (tensor_core_path(desc) && desc->c_hidden == 64)) && chunks_ok)
+    // (c = 128 with a ragged last column chunk stays there too: the tensor map gives every chunk the extent col_chunk, so
+    // the TMA stores would write past the last column, where the warp-MMA kernel leaves the caller's memory alone)
+    const bool whole_chunks = (a->col_chunk >= a->cols || a->cols % a->col_chunk == 0) &&
+                              (b->col_chunk >= b->cols || b->cols % b->col_chunk == 0);
+    if ((narrow_tensor_core_path(desc) || (tensor_core_path(desc) && desc->c_hidden == 64 && whole_chunks)) && chunks_ok)
         return run_narrow_tm1(desc, z, mask, w, a, b, st, status);
     const void* mats[4] = {w->w_left, w->w_left_gate, w->w_right, w->w_right_gate};
     if (wmma_ok(desc, mats, 4)) return run_wmma_tm1(desc, z, mask, w, a, b, st);

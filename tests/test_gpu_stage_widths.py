@@ -224,3 +224,25 @@ def test_stage3_with_the_layernorms_in_place_on_request(dev, c, h, residual):
     # fp32 sums in another order differ by about 1e-6 of the value and a bf16 step is 4e-3 of it: a few in ten thousand of
     # the roundings of LN(x), and of the outputs, go the other way
     assert (asked != plain).float().mean() <= 0.02
+
+
+@pytest.mark.parametrize("outgoing", [True, False], ids=["outgoing", "incoming"])
+def test_stage1_leaves_what_is_past_a_ragged_last_chunk_alone(dev, outgoing):
+    """c = 128, h = 64, column chunks of 64 over 100 columns: the last chunk holds 36."""
+    from miniworld_engine_b200 import read_status, stages as S
+    B, N = 1, 100
+    kw = weights_dict(O.make_weights(128, 81, affine="random", h=64), torch.bfloat16, dev)
+    z = O.make_input(B, N, 128, 82).bfloat16().to(dev)
+    outs = []
+    for layout in ({}, dict(col_chunk=64)):
+        a, b = (S.alloc_planes(B * 64, N, N, torch.bfloat16, dev, fill=float("nan"), **layout) for _ in range(2))
+        S.tm1(z, None, kw, a, b, outgoing=outgoing)
+        outs.append([S.planes_to_dense(s).float().cpu() for s in (a, b)])
+        if layout:
+            for s in (a, b):
+                last = s.buf[s.chunk_stride:].view(64, N, s.pitch)
+                assert torch.isnan(last[..., N - 64:]).all()
+    assert read_status(dev)[0] == 0
+    for ref, got in zip(*outs):
+        assert not torch.isnan(got).any()
+        assert O.rel_rms(got, ref) <= 4e-3      # two kernels, the same rounding points
