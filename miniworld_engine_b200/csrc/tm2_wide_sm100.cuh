@@ -27,8 +27,10 @@
 //                 rows per thread and a halving butterfly over the 8 lanes that share the positions
 //   warps 8..19   epilogue: warp = (TMEM lane quarter, third of the eight 32-channel pieces): TMEM -> statistics ->
 //                 gate -> (* scale) (+ residual) -> bf16 -> the warp's own [32 positions][32 channels] box -> TMA store
-// Before the first tile warps 4..11 fold gamma and 1/2 into the weights; the per-channel (rowsum, bias) pairs are
-// written to both CTAs.
+// Before the first tile warps 4..19 fold gamma and 1/2 into the weights, Wg while Wo is still on its way, while the tile's z
+// slices arrive; the per-channel (rowsum, bias) pairs are written to both CTAs.  With one tile per CTA that start is a third
+// of the stage: with eight folding warps and z slices requested only after the fold the block took 1.5 us longer (N = 64
+// 40.1 -> 38.6 us without the residual, 40.6 -> 39.0 with it; N = 256 117.1 -> 114.7 and 121.2 -> 117.8).
 //
 // mbarriers (full, empty, acc_full, stat in each CTA; ready and acc_empty used in the leader only):
 //   full[s]       this CTA's slice landed        ready[s]      2 arrivals: both CTAs' slices landed
@@ -84,8 +86,8 @@ tm2_wide_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     float4* sConst = reinterpret_cast<float4*>(smem + kW2OffConst);
     float4* sStat = reinterpret_cast<float4*>(smem + kW2OffStat);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kW2OffBars);
-    uint64_t* w_full = bars;
-    uint64_t* full = bars + 1;                // [slots]
+    uint64_t* w_full = bars;                  // [2] Wg, Wo half landed
+    uint64_t* full = bars + 2;                // [slots]
     uint64_t* ready = full + kW2Slots;        // [slots] leader
     uint64_t* empty = ready + kW2Slots;       // [slots]
     uint64_t* acc_full = empty + kW2Slots;
@@ -93,7 +95,7 @@ tm2_wide_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     uint64_t* stat = acc_empty + 1;           // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stat + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    static_assert((5 + 3 * kW2Slots) * 8 + 8 <= 256, "barrier block too small");
+    static_assert((6 + 3 * kW2Slots) * 8 + 8 <= 256, "barrier block too small");
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -101,7 +103,8 @@ tm2_wide_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     const bool is_leader = rank == 0;
 
     if (threadIdx.x == 0) {
-        mbar_init(w_full, 1);
+        mbar_init(&w_full[0], 1);
+        mbar_init(&w_full[1], 1);
         for (int s = 0; s < kW2Slots; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&ready[s], 2);
@@ -142,29 +145,50 @@ tm2_wide_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         b = br / p.rows;
     };
 
-    if (warp == 0 && lane == 0) {
-        mbar_arrive_expect_tx(w_full, 8 * kW2WSub);
-        for (int ks = 0; ks < 4; ++ks) {
-            tma_load_2d(sW + ks * kW2WSub, &tmWg, w_full, ks * 64, (int)rank * 128);
-            tma_load_2d(sW + (4 + ks) * kW2WSub, &tmWo, w_full, ks * 64, (int)rank * 128);
+    // slice u of this CTA (slice j of its tile) into slot u % kW2Slots
+    auto load_slice = [&](uint32_t u, int j, int b, int r, int j0) {
+        const int s = u % kW2Slots;
+        mbar_arrive_expect_tx(&full[s], kW2SlotBytes);
+        uint8_t* dst = sSlot + s * kW2SlotBytes;
+        if (j < 4) {
+            tma_load_4d(dst, &tmZ, &full[s], j * 64, j0, r, b);
+        } else {
+            // tri planes viewed as (column, row, plane, chunk): 64 columns x 64 planes per box
+            const int plane = b * kW2C + (j - 4) * 64;
+            tma_load_4d(dst, &tmTri, &full[s], j0, r, plane, 0);
+            tma_load_4d(dst + kW2SlotBytes / 2, &tmTri, &full[s], j0 + 64, r, plane, 0);
         }
+    };
+    if (warp == 0 && lane == 0) {
+        mbar_arrive_expect_tx(&w_full[0], 4 * kW2WSub);
+        for (int ks = 0; ks < 4; ++ks) tma_load_2d(sW + ks * kW2WSub, &tmWg, &w_full[0], ks * 64, (int)rank * 128);
+        mbar_arrive_expect_tx(&w_full[1], 4 * kW2WSub);
+        for (int ks = 0; ks < 4; ++ks) tma_load_2d(sW + (4 + ks) * kW2WSub, &tmWo, &w_full[1], ks * 64, (int)rank * 128);
+        // the first tile's z slices fill the empty ring while the weights are folded
+        int b, r, j0;
+        place(cluster_id, b, r, j0);
+        for (int j = 0; j < kW2Slots; ++j) load_slice(j, j, b, r, j0);
     }
     __syncwarp();
-    if (warp >= 4 && warp < 12) {
-        // thread: matrix m (0: Wg with LN_in, 1: Wo with LN_out), row n of this CTA's half
-        const int e = threadIdx.x - 128, m = e >> 7, n = e & 127;
-        if (mbar_wait<true>(w_full, 0, abort_flag, p.status, kStageIdTm2, 1150)) {
-            float s_, b_;
-            fold_row_smem(sW + m * 4 * kW2WSub, kW2WSub, n, m == 0 ? p.gamma_in : p.gamma_out,
-                          m == 0 ? p.beta_in : p.beta_out, 4, s_, b_);
-            const int ch = (int)rank * 128 + n;
-            const uint32_t dst = smem_u32(reinterpret_cast<float*>(&sConst[m * 128 + (ch >> 1)]) + (ch & 1));
-            for (uint32_t k = 0; k < 2; ++k) {
-                const uint32_t a = map_to_cta(dst, k);
-                st_cluster_f32(a, s_);
-                st_cluster_f32(a + 8, b_);
-            }
+    if (warp >= 4) {
+        // two threads per row: matrix m (0: Wg with LN_in, 1: Wo with LN_out), row n of this CTA's half, half of the K slices
+        // (16 rows and both K halves in a warp: eight lanes of a quarter warp on eight rows of one K slice)
+        const int w = warp - 4, m = w >> 3, n = 16 * (w & 7) + (lane & 15), kh = lane >> 4;
+        float s_ = 0.f, b_ = 0.f;
+        const bool landed = mbar_wait<true>(&w_full[m], 0, abort_flag, p.status, kStageIdTm2, 1150);
+        if (landed) {
+            fold_row_smem(sW + (4 * m + 2 * kh) * kW2WSub, kW2WSub, n, (m == 0 ? p.gamma_in : p.gamma_out) + 128 * kh,
+                          (m == 0 ? p.beta_in : p.beta_out) + 128 * kh, 2, s_, b_);
             fence_proxy_async_smem();      // folded weights -> visible to the UMMA (async proxy)
+        }
+        __syncwarp();
+        s_ += __shfl_xor_sync(0xffffffffu, s_, 16);
+        b_ += __shfl_xor_sync(0xffffffffu, b_, 16);
+        if (landed) {                      // K half kh writes the pair's sums to CTA kh
+            const int ch = (int)rank * 128 + n;
+            const uint32_t a = map_to_cta(smem_u32(reinterpret_cast<float*>(&sConst[m * 128 + (ch >> 1)]) + (ch & 1)), (uint32_t)kh);
+            st_cluster_f32(a, s_);
+            st_cluster_f32(a + 8, b_);
         }
     }
     __syncwarp();
@@ -173,27 +197,18 @@ tm2_wide_sm100_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
-            uint32_t u = 0;
+            uint32_t u = kW2Slots;         // slices 0 .. 3 of the first tile are on their way
             bool ok = true;
             for (int pt = cluster_id; ok && pt < total_pairs; pt += num_clusters) {
                 int b, r, j0;
                 place(pt, b, r, j0);
-                for (int j = 0; j < 8; ++j, ++u) {
+                for (int j = pt == cluster_id ? kW2Slots : 0; j < 8; ++j, ++u) {
                     const int s = u % kW2Slots;
                     if (!mbar_wait<true>(&empty[s], ((u / kW2Slots) & 1u) ^ 1u, abort_flag, p.status, kStageIdTm2, 1100 + s)) {
                         ok = false;
                         break;
                     }
-                    mbar_arrive_expect_tx(&full[s], kW2SlotBytes);
-                    uint8_t* dst = sSlot + s * kW2SlotBytes;
-                    if (j < 4) {
-                        tma_load_4d(dst, &tmZ, &full[s], j * 64, j0, r, b);
-                    } else {
-                        // tri planes viewed as (column, row, plane, chunk): 64 columns x 64 planes per box
-                        const int plane = b * kW2C + (j - 4) * 64;
-                        tma_load_4d(dst, &tmTri, &full[s], j0, r, plane, 0);
-                        tma_load_4d(dst + kW2SlotBytes / 2, &tmTri, &full[s], j0 + 64, r, plane, 0);
-                    }
+                    load_slice(u, j, b, r, j0);
                 }
             }
         }
