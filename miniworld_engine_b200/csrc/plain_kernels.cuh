@@ -359,19 +359,14 @@ __global__ void __launch_bounds__(kPlainThreads, 2) plain_contract_kernel(PlaneV
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r >= v.rows || k >= K) return x;
         const T* base = static_cast<const T*>(v.base);
-        if (quads) {
-            // pitch (and a column chunk) is a multiple of 4: the quad lies inside the row's storage, but what is past
-            // the last column is never used
+        if (quads && k + 3 < K) {
             x = load_f4(base + v.offset(plane, r, k));
-        } else {
+        } else {                      // nothing past the last column is read: the caller's memory may end there
             x.x = load_f<T>(base + v.offset(plane, r, k));
             if (k + 1 < K) x.y = load_f<T>(base + v.offset(plane, r, k + 1));
             if (k + 2 < K) x.z = load_f<T>(base + v.offset(plane, r, k + 2));
             if (k + 3 < K) x.w = load_f<T>(base + v.offset(plane, r, k + 3));
         }
-        if (k + 1 >= K) x.y = 0.f;
-        if (k + 2 >= K) x.z = 0.f;
-        if (k + 3 >= K) x.w = 0.f;
         return x;
     };
     auto fetch = [&](int k0) {
