@@ -136,8 +136,8 @@ def test_cfg4_outgoing_bf16_b2_n512_dpair_sweep(c, dev):
     (64, 2, 70, "tail7"), (256, 1, 65, "rand5"), (48, 1, 33, None), (32, 1, 130, "tail20"), (208, 1, 20, "tail3"),
 ], ids=["c64", "c256", "c48", "c32", "c208"])
 def test_bf16_other_widths_take_the_warp_mma_kernels(dev, c, B, N, mask_kind, outgoing):
-    """bf16 with c != 128 (a multiple of 16): stages 1 and 3 run on the warp-MMA kernels.  Checked
-    against the oracle and, stage by stage on a row slab (rows < N, row0 > 0), against the scalar
+    """bf16 with c != 128 (a multiple of 16): stages 1 and 3 run on the warp-MMA kernels, at c = 64 and 256 on
+    the tcgen05 kernels of those widths.  Checked against the oracle and, stage by stage on a row slab (rows < N, row0 > 0), against the scalar
     CUDA-core kernels, which round at the same points."""
     from miniworld_engine_b200 import stages as S
     from tests._util import weights_dict

@@ -59,9 +59,10 @@ def test_stage1_matches_the_cuda_core_kernel(dev, c, B, N, mask_kind, layout, ou
     (1, 1, "z", False), (2, 33, None, False), (1, 128, "z", True), (1, 129, None, True), (3, 127, "z", False),
     (1, 255, "other", False), (1, 300, "z", True), (3, 130, "z", True), (1, 385, None, False)])
 def test_stage3_against_64_bits(dev, c, h, B, N, residual, scale):
-    """The folded last stage, and what takes over where it does not apply (another residual, LayerNorm vectors that
-    are not 16-byte aligned), against the stage in 64 bits on the same bf16 operands."""
+    """The folded last stage, with LayerNorm vectors at any float address, and what takes over for another residual,
+    against the stage in 64 bits on the same bf16 operands."""
     from miniworld_engine_b200 import _lib, read_status, stages as S
+    from miniworld_engine_b200.functional import _status_words
     import ctypes as C
     w = O.make_weights(c, 41, affine="random", h=h).to(torch.bfloat16)
     kw = weights_dict(w, torch.bfloat16, dev)
@@ -93,10 +94,10 @@ def test_stage3_against_64_bits(dev, c, h, B, N, residual, scale):
         ws, _ = S._weights_struct(c, z.dtype, device=dev, c_hidden=h, c_proj=h, **k)
         desc = _lib.make_desc(B, N, c, c_hidden=h, dtype=_lib.DTYPE_BF16, direction=_lib.OUTGOING, eps_in=w.eps_in,
                               eps_out=w.eps_out, drop_scale=None if dsd is None else dsd.data_ptr())
-        out = torch.empty_like(zd)
+        out = torch.full_like(zd, float("nan"))
         _lib.check(lib.trimul_b200_tm2(C.byref(desc), zd.data_ptr(), C.byref(t.struct()), C.byref(ws), out.data_ptr(),
                                        None if rd is None else rd.data_ptr(),
-                                       torch.cuda.current_stream(dev).cuda_stream, None), "tm2")
+                                       torch.cuda.current_stream(dev).cuda_stream, _status_words(dev).data_ptr()), "tm2")
         y = out.cpu().double()
         ref = upd if res is None else upd + d64(res)
         errs.append(float((y - ref).norm() / ref.norm()))
@@ -104,6 +105,40 @@ def test_stage3_against_64_bits(dev, c, h, B, N, residual, scale):
     # roundings to bf16 (1.1e-3 rms each): the folded weights or the normalised operands, twice; the output, with a
     # scale and a residual once more each; the hardware tanh adds 2.5e-4 of the gate
     assert max(errs) <= 5e-3, errs
+
+
+@pytest.mark.parametrize("residual", [False, True], ids=["bare", "residual"])
+@pytest.mark.parametrize("c,h", [(64, 64), (128, 64), (128, 128), (128, 256), (256, 256)])
+def test_stage3_of_a_row_slab_is_that_part_of_the_whole(dev, c, h, residual):
+    """Rows 37 .. 126 of 200 with a dropout scale, whose tiles are walked in column order (rows != N): the same bits."""
+    from miniworld_engine_b200 import _lib, read_status, stages as S
+    from miniworld_engine_b200.functional import _status_words
+    import ctypes as C
+    B, N, row0, rows = 2, 200, 37, 90
+    kw = weights_dict(O.make_weights(c, 91, affine="random", h=h), torch.bfloat16, dev)
+    g = torch.Generator().manual_seed(92)
+    z = torch.randn(B, N, N, c, generator=g).bfloat16().to(dev)
+    tri = torch.randn(B * h, N, N, generator=g).bfloat16().to(dev)
+    ds = ((torch.rand(B, 1, N, c, generator=g) > 0.25).float() / 0.75).bfloat16().to(dev)
+    ws, _ = S._weights_struct(c, z.dtype, device=dev, c_hidden=h, c_proj=h, **kw)
+
+    def run(first, count):
+        zs = z[:, first:first + count].contiguous()
+        t = S.alloc_planes(B * h, count, N, torch.bfloat16, dev, fill=float("nan"))
+        S.dense_to_planes(t, tri[:, first:first + count])
+        desc = _lib.make_desc(B, N, c, c_hidden=h, dtype=_lib.DTYPE_BF16, direction=_lib.OUTGOING, rows=count, row0=first,
+                              drop_scale=ds.data_ptr())
+        out = torch.full_like(zs, float("nan"))
+        _lib.check(_lib.load().trimul_b200_tm2(C.byref(desc), zs.data_ptr(), C.byref(t.struct()), C.byref(ws), out.data_ptr(),
+                                               zs.data_ptr() if residual else None,
+                                               torch.cuda.current_stream(dev).cuda_stream,
+                                               _status_words(dev).data_ptr()), "tm2")
+        return out
+
+    whole, slab = run(0, N), run(row0, rows)
+    assert read_status(dev)[0] == 0
+    assert not torch.isnan(whole.float()).any()
+    assert torch.equal(slab, whole[:, row0:row0 + rows])
 
 
 @pytest.mark.parametrize("single_cta", [False, True], ids=["pair", "lone"])
