@@ -37,7 +37,7 @@ import torch.nn as nn
 from . import _lib
 from .functional import (_dtype_code, _mask_bytes, _on_device, _pinned_weights, _plain, _require_cuda, _require_no_grad,
                          _status_words, _stream_handle, _workspace)
-from .module import PinnedLayerNormParams, _lecun_trunc_normal_, _param, _sub
+from .module import PinnedLayerNormParams, _lecun_trunc_normal_, _param, _submodules
 
 __all__ = ["bidir_trimul_forward", "bidirectional_triangle_multiplicative_update_b200",
            "BidirectionalTriangleMultiplicationB200"]
@@ -170,14 +170,15 @@ class BidirectionalTriangleMultiplicationB200(nn.Module):
 
     def _block_no_grad(self, pair, mask, add_residual, plain_kernels) -> torch.Tensor:
         """The body of ``block``, apart from it so that an override of ``block`` is not entered a second time."""
-        ln_in, ln_out = _sub(self, "ln_pair"), _sub(self, "ln_out")
+        m = _submodules(self, BidirectionalTriangleMultiplicationB200)
+        ln_in, ln_out = m["ln_pair"], m["ln_out"]
         return bidir_trimul_forward(
             pair, mask,
             ln_in_weight=_param(ln_in, "weight"), ln_in_bias=_param(ln_in, "bias"),
-            w_left=_param(_sub(self, "to_left"), "weight"), w_left_gate=_param(_sub(self, "to_left_gate"), "weight"),
-            w_right=_param(_sub(self, "to_right"), "weight"), w_right_gate=_param(_sub(self, "to_right_gate"), "weight"),
+            w_left=_param(m["to_left"], "weight"), w_left_gate=_param(m["to_left_gate"], "weight"),
+            w_right=_param(m["to_right"], "weight"), w_right_gate=_param(m["to_right_gate"], "weight"),
             ln_out_weight=_param(ln_out, "weight"), ln_out_bias=_param(ln_out, "bias"),
-            w_gate=_param(_sub(self, "to_gate"), "weight"), w_out=_param(_sub(self, "to_out"), "weight"),
+            w_gate=_param(m["to_gate"], "weight"), w_out=_param(m["to_out"], "weight"),
             eps_in=ln_in.eps, eps_out=ln_out.eps,
             add_residual=add_residual, plain_kernels=plain_kernels)
 

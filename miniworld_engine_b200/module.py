@@ -64,13 +64,16 @@ def _param(module: nn.Module, name: str) -> torch.Tensor:
     return t
 
 
-def _sub(module: nn.Module, name: str) -> nn.Module:
-    """``getattr(module, name)``; a registered submodule that neither the class nor the instance shadows is read from the
-    module's own table."""
-    sub = module._modules.get(name)
-    if sub is None or name in module.__dict__ or hasattr(type(module), name):
-        return getattr(module, name)
-    return sub
+_SUBMODULES = ("ln_pair", "to_left", "to_left_gate", "to_right", "to_right_gate", "ln_out", "to_gate", "to_out")
+
+
+def _submodules(module: nn.Module, cls: type) -> dict:
+    """``{name: getattr(module, name)}`` of a block's submodules: the module's own table where nothing can shadow it (no subclass,
+    and no attribute of one of these names on the instance or the class)."""
+    if (type(module) is cls and module.__dict__.keys().isdisjoint(_SUBMODULES)
+            and cls.__dict__.keys().isdisjoint(_SUBMODULES)):
+        return module._modules
+    return {name: getattr(module, name) for name in _SUBMODULES}
 
 
 _PLAIN_TYPES = (nn.Linear, PinnedLayerNormParams)
@@ -131,14 +134,15 @@ class TriangleMultiplicationB200(nn.Module):
 
     def _block_no_grad(self, pair, mask, residual, plain_kernels, drop_scale) -> torch.Tensor:
         """The body of ``block``, apart from it so that an override of ``block`` is not entered a second time."""
-        ln_in, ln_out = _sub(self, "ln_pair"), _sub(self, "ln_out")
+        m = _submodules(self, TriangleMultiplicationB200)
+        ln_in, ln_out = m["ln_pair"], m["ln_out"]
         return F_b200.trimul_forward(
             pair, mask, outgoing=self.outgoing,
             ln_in_weight=_param(ln_in, "weight"), ln_in_bias=_param(ln_in, "bias"),
-            w_left=_param(_sub(self, "to_left"), "weight"), w_left_gate=_param(_sub(self, "to_left_gate"), "weight"),
-            w_right=_param(_sub(self, "to_right"), "weight"), w_right_gate=_param(_sub(self, "to_right_gate"), "weight"),
+            w_left=_param(m["to_left"], "weight"), w_left_gate=_param(m["to_left_gate"], "weight"),
+            w_right=_param(m["to_right"], "weight"), w_right_gate=_param(m["to_right_gate"], "weight"),
             ln_out_weight=_param(ln_out, "weight"), ln_out_bias=_param(ln_out, "bias"),
-            w_gate=_param(_sub(self, "to_gate"), "weight"), w_out=_param(_sub(self, "to_out"), "weight"),
+            w_gate=_param(m["to_gate"], "weight"), w_out=_param(m["to_out"], "weight"),
             eps_in=ln_in.eps, eps_out=ln_out.eps,
             residual=residual, plain_kernels=plain_kernels, drop_scale=drop_scale)
 
