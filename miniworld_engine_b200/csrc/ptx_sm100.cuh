@@ -450,14 +450,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
 
-// sigmoid(x) = 0.5 * tanh(0.5 x) + 0.5 with the hardware tanh: one MUFU operation per value
-// (absolute error ~5e-4 of tanh.approx, i.e. ~2.5e-4 on the gate — a quarter of a bf16 ulp at 1).
-__device__ __forceinline__ float sigmoid_fast(float x) {
-    float t;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * x));
-    return fmaf(0.5f, t, 0.5f);
-}
-
 // ---------------------------------------------------------------------------------------
 // CTA pairs (clusters of two, tcgen05 cta_group::2).  No TMA multicast is used anywhere: a pair's
 // loads land in the issuing CTA and only their completion is signalled across the pair.
@@ -580,18 +572,17 @@ __device__ __forceinline__ float tanh_fast(float x) {
 // p * sigmoid(g) from HALVED inputs hp = p/2, hg = g/2:  p*sigmoid(g) = hp*tanh(hg) + hp.
 // The kernels halve the weight matrices once in shared memory (exact in bf16), so the
 // accumulators already hold hp and hg and the gate costs one MUFU and one FMA per value.
-__device__ __forceinline__ float gate_from_halves(float hp, float hg) { return fmaf(hp, tanh_fast(hg), hp); }
 // two gates at once, result rounded to a bf16x2 word
 __device__ __forceinline__ uint32_t gate2_bf16(float hp0, float hg0, float hp1, float hg1) {
     const f32x2 hp = f2_pack(hp0, hp1);
     return f2_to_bf16x2(f2_fma(hp, f2_pack(tanh_fast(hg0), tanh_fast(hg1)), hp));
 }
 
-// p * sigmoid(g) for two values from halves, rounded to a bf16x2 word.  kFp32: the gate to 1e-6 of its own size (1e-5 at
-// g = -80), as p/2 times 2 / (1 + 2^(-2 log2(e) g/2)).  tanh.approx is off by up to 2.5e-4 of the gate's FULL scale, which
-// leaves nothing of a nearly shut gate (sigmoid(-8) = 3.4e-4); the fp32 form takes two MUFU operations instead of one and is
-// for the widths whose gates were evaluated in fp32 before they had a tcgen05 kernel.  (Flush to zero: a power below 2^-126
-// does not show beside 1; gates below 2^-126, at g < -87, become 0.)
+// p * sigmoid(g) for two values from halves, rounded to a bf16x2 word.  The tanh form is off by up to 4e-6 of the gate's FULL
+// scale (measured over logits from -90 to 12): nothing beside a bf16 step of an open gate, but 0.3 % of a gate at g = -8
+// (sigmoid 3.4e-4), 1.5 % at -13, 26 % at -15, and below -17 the gate is 0.  kFp32: p/2 times 2 / (1 + 2^(-2 log2(e) g/2)),
+// off by 5e-7 of the gate's own size at g = -8, 1e-6 at -20, 4e-6 at -87 (0 below: flush to zero), with two MUFU operations
+// instead of one; for the widths whose gates were evaluated in fp32 before they had a tcgen05 kernel.
 template <bool kFp32>
 __device__ __forceinline__ uint32_t gate_halves_bf16(f32x2 hp, f32x2 hg) {
     float g0, g1;
