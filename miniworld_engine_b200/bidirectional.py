@@ -21,7 +21,7 @@ bf16 with ``d = h = 128`` takes the tensor-core kernels in every stage.  ``d_hid
 (``h`` a multiple of 8, ``2h <= 256``) is served too: stage 1 then runs on the tensor-core kernel of
 64 hidden channels (``h = 64`` and ``d`` 64 or 128), else on the warp-MMA kernel (widths that are multiples
 of 16) or the CUDA-core kernel, the contraction stays on the tensor cores for bf16, and stage 3 does when ``d = 128`` and
-``2h`` is 128 or 256.  fp32 takes the CUDA-core kernels throughout.
+``2h`` is 64, 128 or 256, or ``d = 2h`` is 64 or 256.  fp32 takes the CUDA-core kernels throughout.
 
 ``bidirectional_triangle_multiplicative_update_b200`` is the same call under the argument names of
 the reference's functional op (``kernels/trimul_inproj/whole_op.py:243-262``).

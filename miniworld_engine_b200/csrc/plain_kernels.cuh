@@ -10,11 +10,12 @@
 // chunked addressing of trimul_planes, so they work on gathered multi-GPU operands unchanged.
 //
 // What bounds them: FP32 FMA issue (148 SMs x 128 lanes, 74 TFLOP/s at 1.965 GHz).  So each stage is a
-// register-tiled matrix product: 256 threads, a thread owns TM positions x 8 columns (16 with the
-// contraction's TM = 8 counted as 8 x 8), both operands lie K-major in shared memory as [k][position]
-// and [k][column], and one K step costs three or four 16-byte shared-memory reads per 8 TM FMAs.  Eight
-// lanes of a warp walk positions and four walk columns, so a position fragment of a warp is one 128-byte
-// wavefront.  Every output is still ONE fma chain over ascending k: the rounding of the products
+// register-tiled matrix product: 256 threads, both operands K-major in shared memory as [k][position] and
+// [k][column].  A thread owns TM positions x 8 columns in stage 1 (four of a projection, four of its gate), TM x TM outputs in
+// the contraction and TM positions x 4 columns in stage 3 (of the gate, then of the projection): one K step at TM = 8
+// costs four 16-byte shared-memory reads per 64 FMAs in stages 1 and 2, three per 32 in stage 3, which is why that
+// stage's load/store pipe is the busiest.  Eight lanes of a warp walk positions and four walk columns, so a
+// position fragment of a warp is one 128-byte wavefront.  Every output is still ONE fma chain over ascending k: the rounding of the products
 // is what a plain dot product gives; the FMAs are the packed two-lane form.
 // Measured (fp32, B = 1, N = 256, c = 128; before: one output channel per thread, 8 positions, weights read
 // from global memory with a stride of c): stage 1 2215 -> 302 us, contraction 646 -> 143, stage 3 1206 -> 193,

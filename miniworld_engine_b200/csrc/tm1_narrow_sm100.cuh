@@ -14,7 +14,7 @@
 // had expf, the fp32 form, which keeps the bits of nearly shut gates.  It costs 1.8 us of a call at N = 512).
 //
 // What bounds it: HBM (c = 64: z once, a and b once).  LayerNorm and epilogue have the form of the CTA-pair
-// kernel (tm1_pair_sm100.cuh): eight lanes per LayerNorm row with every value read once, and sixteen
+// kernel (tm1_pair_sm100.cuh): four lanes (c = 64) or eight (c = 128) per LayerNorm row with every value read once, and sixteen
 // epilogue warps that store their own boxes, two tiles in flight, instead of one thread per row and two groups
 // behind block-wide barriers.  Measured: c = 64, B = 2, N = 512: 1.35 us per tile and CTA on the timeline
 // (48 KB of traffic: 5.3 TB/s over the chip), 2.1 us before; c = 128 (K = 128, 64 KB per tile): 2.4 us, paced by the

@@ -95,7 +95,6 @@ constexpr int kG2EpiBarrier = 4;        // 4: channels 0..63, 5: channels 64..12
 
 struct Tm2FoldParams {
     Tm2Params base;
-    int residual_is_z;    // add the z tile to the result (the block's `pair + update` form)
     const __nv_bfloat16* drop_scale;   // [B, 1, N, c] row-broadcast multiplier of the block output
                                        // (module.py:332-337), applied before the residual; or null
 };

@@ -212,13 +212,13 @@ bool tensor_core_path(const trimul_desc* d) {
     return d->dtype == TRIMUL_DTYPE_BF16 && d->c == 128 && (d->flags & TRIMUL_FLAG_PLAIN_KERNELS) == 0;
 }
 
-// bf16 with c = h = 256: the streamed-weight tensor-core kernels of stages 1 and 3
+// bf16 with c = h = 256: stage 1 with streamed weights, stage 3 on CTA pairs with resident ones
 bool wide_tensor_core_path(const trimul_desc* d) {
     return d->dtype == TRIMUL_DTYPE_BF16 && d->c == 256 && d->c_hidden == 256 &&
            (d->flags & TRIMUL_FLAG_PLAIN_KERNELS) == 0;
 }
 
-// bf16 with c = h = 64: the stacked-operand tensor-core kernels of stages 1 and 3
+// bf16 with c = h = 64: stage 1 with both sides' weights in one operand, stage 3 folded (or, for another residual, in place)
 bool narrow_tensor_core_path(const trimul_desc* d) {
     return d->dtype == TRIMUL_DTYPE_BF16 && d->c == 64 && d->c_hidden == 64 &&
            (d->flags & TRIMUL_FLAG_PLAIN_KERNELS) == 0;
@@ -664,7 +664,6 @@ int run_fold_tm2(const trimul_desc* d, const void* z, const trimul_planes* tri, 
     if (!encode_planes(&tmTri, *tri, d->B * kH, 64, 1, G2Layout<kC, kH, false>::kSlotCh)) return TRIMUL_E_CUDA;
     Tm2FoldParams fp;
     fp.base = tm2_params(d, w, residual, status);
-    fp.residual_is_z = residual != nullptr;
     fp.drop_scale = static_cast<const __nv_bfloat16*>(desc_drop_scale(d));
     const int grid = fp.base.total_tiles < sm_count() ? fp.base.total_tiles : sm_count();
     CUtensorMap tmScale = tmZ;
