@@ -884,8 +884,8 @@ __device__ __forceinline__ void ln_load_affine_quad(f32x2 (&gb)[16], const float
 }
 
 // gamma and beta of a lane's channels for ln_rows_warp, from global memory: lane chunk j = lane & 7 owns
-// channels [64 s + 8 j, 64 s + 8 j + 8) of every sub-tile s.  4-byte loads, once per thread and launch: the vectors may lie at
-// any float address (a view into a flat parameter buffer).
+// channels [64 s + 8 j, 64 s + 8 j + 8) of every sub-tile s.  4-byte loads: the vectors may lie at any float address (a
+// view into a flat parameter buffer).
 template <int kSub>
 __device__ __forceinline__ void ln_load_affine(f32x2 (&gb)[8 * kSub], const float* gamma, const float* beta, int lane) {
 #pragma unroll
@@ -895,6 +895,20 @@ __device__ __forceinline__ void ln_load_affine(f32x2 (&gb)[8 * kSub], const floa
             const int ch = 64 * s + 8 * (lane & 7) + 2 * k;
             gb[4 * s + k] = f2_pack(__ldg(gamma + ch), __ldg(gamma + ch + 1));
             gb[4 * kSub + 4 * s + k] = f2_pack(__ldg(beta + ch), __ldg(beta + ch + 1));
+        }
+}
+
+// The same from shared memory: gamma[64 kSub], then beta[64 kSub], 16-byte aligned.
+template <int kSub>
+__device__ __forceinline__ void ln_load_affine_smem(f32x2 (&gb)[8 * kSub], const float* affine, int lane) {
+#pragma unroll
+    for (int v = 0; v < 2; ++v)
+#pragma unroll
+        for (int s = 0; s < kSub; ++s) {
+            const ulonglong2* p = reinterpret_cast<const ulonglong2*>(affine + 64 * (kSub * v + s) + 8 * (lane & 7));
+            const ulonglong2 lo = p[0], hi = p[1];
+            gb[4 * (kSub * v + s)] = lo.x; gb[4 * (kSub * v + s) + 1] = lo.y;
+            gb[4 * (kSub * v + s) + 2] = hi.x; gb[4 * (kSub * v + s) + 3] = hi.y;
         }
 }
 
