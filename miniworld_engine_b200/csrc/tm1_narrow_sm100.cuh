@@ -18,7 +18,7 @@
 // epilogue warps that store their own boxes, two tiles in flight, instead of one thread per row and two groups
 // behind block-wide barriers.  Measured: c = 64, B = 2, N = 512: 1.35 us per tile and CTA on the timeline
 // (48 KB of traffic: 5.3 TB/s over the chip), 2.1 us before; c = 128 (K = 128, 64 KB per tile): 2.4 us, paced by the
-// LayerNorm of 128 rows x 128 channels.
+// LayerNorm of 128 rows x 128 channels (2.5 with the fp32 gates, from N = 448 30.5 -> 32.1 us).
 //
 // Persistent kernel, one CTA per SM, 832 threads, 128-position tiles:
 //   warp 0        TMA producer: the weights once, then z tiles

@@ -849,8 +849,8 @@ int trimul_b200_tm1(const trimul_desc* desc, const void* z, const uint8_t* mask,
     if (tensor_core_path(desc) && desc->c_hidden == 128 && chunks_ok)
         return run_fast_tm1(desc, z, mask, w, a, b, st, status);
     if (wide_tensor_core_path(desc) && chunks_ok) return run_wide_tm1(desc, z, mask, w, a, b, st, status);
-    // h = 64: the stacked-operand kernel (c = 128, bidirectional N = 320: 23 us a call,
-    // 159 on the warp-MMA kernel, which keeps the other widths)
+    // h = 64: the stacked-operand kernel (c = 128, back to back: N = 64 8.1 us, 18.7 on the warp-MMA kernel, which keeps
+    // the other widths; N = 320 19.7 and 143, N = 448 32.6 and 296)
     // (c = 128 with a ragged last column chunk stays there too: the tensor map gives every chunk the extent col_chunk, so
     // the TMA stores would write past the last column, where the warp-MMA kernel leaves the caller's memory alone)
     const bool whole_chunks = (a->col_chunk >= a->cols || a->cols % a->col_chunk == 0) &&
@@ -972,8 +972,8 @@ int trimul_b200_tm2(const trimul_desc* desc, const void* z, const trimul_planes*
                              : run_inplace_tm2(desc, z, tri, w, out, residual, st, status);
         if (desc->c_hidden == 256 && folded_ok) return run_fold_tm2<128, 256>(desc, z, tri, w, out, residual, st, status);
     }
-    // h = 64 (in the step, c = 64, B = 2, N = 512: 53 us, 74 with both LayerNorms in place; c = 128, N = 448: 42 us, 345 on the
-    // warp-MMA kernel)
+    // h = 64 (in the step, c = 64, B = 2, N = 512: 53 us, 74 with both LayerNorms in place; c = 128 back to back, N = 64: 8.5 us, 23.4
+    // on the warp-MMA kernel, N = 448: 39.7 and 349)
     if (folded_ok && desc->c_hidden == 64) {
         if (tensor_core_path(desc)) return run_fold_tm2<128, 64>(desc, z, tri, w, out, residual, st, status);
         if (narrow_tensor_core_path(desc)) return run_fold_tm2<64, 64>(desc, z, tri, w, out, residual, st, status);
